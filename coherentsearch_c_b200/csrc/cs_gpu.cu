@@ -625,6 +625,7 @@ cs_search_kernel(const SearchArgs args)
 #include "cs_search_ws.cuh"
 #include "cs_interp_tc.cuh"
 #include "cs_search_tma.cuh"
+#include "cs_search_cols.cuh"
 #include "cs_search_f64.cuh"
 #include "cs_collapse.h"
 
@@ -699,6 +700,14 @@ struct GpuSession {
     float2 *d_tc[2];       /* zero-padded spectrum copies (second shifted a bin) */
     size_t c_wtab, c_cchunk, c_tc;
     wsk::TArgs tx;
+    /* register-block kernel (search_cols); use_cols: nharms of its configuration */
+    int use_cols;
+    cols::XArgs cx;
+    int cols_smem;
+    float2 *d_pad;         /* padded spectrum copy */
+    unsigned char *d_ctab;
+    CUtensorMap *d_cmaps;  /* [nh] */
+    size_t c_pad, c_ctab;
     /* interpolation as tensor-core GEMMs (tci::interp_tc), then search_pre */
     int use_tci;
     tci::Band *d_tci_bands;
@@ -791,6 +800,9 @@ static void session_release(GpuSession *S)
     cudaFree(S->d_maps);
     cudaFree(S->d_tc[0]);
     cudaFree(S->d_tc[1]);
+    cudaFree(S->d_pad);
+    cudaFree(S->d_ctab);
+    cudaFree(S->d_cmaps);
     cudaFree(S->d_tci_bands);
     cudaFree(S->d_tci_bimg);
     cudaFree(S->d_tci_hbase);
@@ -863,11 +875,11 @@ static int grow_records(GpuSession *S, unsigned cap)
     return 0;
 }
 
-/* The warp-specialised kernels are compiled for the reference's default
- * search at nharms = 60, 32 and 16: m = 16, decimations 1..6 and the slot
- * layouts and ladder widths of wsk::kCfgDescs, with 32-bit trial positions.
- * Returns the nharms of the matching configuration, or 0. */
-static int ws_config(const CsTables &t, long long total)
+/* The specialised kernels are compiled for the reference's default search at
+ * nharms = 60, 32 and 16: m = 16, decimations 1..6 and the slot layouts and
+ * ladder widths of wsk::kCfgDescs, with 32-bit trial positions.  Returns the
+ * nharms of the matching configuration, or 0. */
+static int ladder_config(const CsTables &t, long long total)
 {
     if (getenv("CS_B200_GENERIC_KERNEL")) return 0;
     if (t.m != wsk::M || t.nslot != 6) return 0;
@@ -889,9 +901,16 @@ static int ws_config(const CsTables &t, long long total)
     double rmax = 0;
     for (int h = 0; h < t.nh; h++) rmax = std::max(rmax, (double)t.harm[h].rfloor0);
     if (rmax + tmax * t.nh * (double)t.pnum / (double)t.q + 64 >= 2147483647.0) return 0;
+    return t.nh;
+}
+
+/* The search_ws kernels' own limits besides: residues in 32 bits and weight
+ * rows at a fixed stride. */
+static int ws_config(const CsTables &t, long long total)
+{
     if ((double)t.q * 5.0 * t.q >= 4294967295.0) return 0;
     for (int h = 0; h < t.nh; h++) if (t.harm[h].P > wsk::WT_STRIDE) return 0;
-    return t.nh;
+    return ladder_config(t, total);
 }
 
 static cudaError_t dev_reserve(void **p, size_t *cap, size_t need);
@@ -1165,6 +1184,146 @@ static bool tma_load(GpuSession *S, const CsTables &t, long long total)
     return tma_prepare(nh) == cudaSuccess;
 }
 
+static const void *cols_fn(int nh)
+{
+    return nh == 60 ? (const void *)cols::search_cols<wsk::Cfg60>
+         : nh == 32 ? (const void *)cols::search_cols<wsk::Cfg32>
+                    : (const void *)cols::search_cols<wsk::Cfg16>;
+}
+
+static void cols_launch(int nh, int grid, int smem, cudaStream_t st, const wsk::Args &w,
+                        const cols::XArgs &x)
+{
+    if (nh == 60)
+        cols::search_cols<wsk::Cfg60><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+    else if (nh == 32)
+        cols::search_cols<wsk::Cfg32><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+    else
+        cols::search_cols<wsk::Cfg16><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+}
+
+/* The geometry of the register-block kernel: columns D trials apart (the
+ * least multiple of 2q and of a phase block, so that a column is a whole,
+ * even number of bins on), windows of 18 or 20 taps a group of 4 trials, box
+ * widths of 2 mod 4 bins (the two column groups' rows then start in opposite
+ * halves of the banks).  Returns false where a window or the shared memory
+ * does not fit: more than a bin a trial (hidr above 1), or a long phase cycle
+ * whose tables would not be worth their size. */
+static bool cols_geometry(const CsTables &t, long long total, long long namps, int max_smem,
+                          cols::Geo &g)
+{
+    using namespace cols;
+    memset(&g, 0, sizeof(g));
+    const long long q = t.q, p = t.pnum;
+    long long D = 2 * q;
+    while (D % TI) D += 2 * q;
+    if (D > 4096 || total < 1) return false;
+    g.nh = t.nh;
+    g.nblk = t.nh / 4;
+    g.D = (int)D;
+    g.npb = (int)(D / TI);
+    const long long ncg = (total + D * TC - 1) / (D * TC);
+    if (ncg * g.npb > (1LL << 30) || ncg * D * TC >= 2147483647LL) return false;
+    g.ncg = (int)ncg;
+    g.ntiles = g.npb * g.ncg;
+    g.total = (int)total;
+    g.nchunks = (int)t.nchunks;
+    int off = 0, bwmax = 0;
+    long long smax = 0;
+    for (int hb = 0; hb < g.nblk; hb++) {
+        int nt = 0, bw = 0;
+        for (int h = 4 * hb + 1; h <= 4 * hb + 4; h++) {
+            const long long d3 = (3 * h * p + q - 1) / q, d12 = (12 * h * p + q - 1) / q;
+            nt = std::max(nt, (int)((16 + 1 + d3 + 1) / 2 * 2));
+            bw = std::max(bw, (int)((d12 + 1) / 2 * 2));
+            const long long s = h * p * (D / q);
+            if (s > (1 << 20)) return false;
+            g.shift[h - 1] = (int)s;
+            smax = std::max(smax, s);
+        }
+        if (nt > 20) return false;
+        bw += nt;
+        if (bw % 4 != 2) bw += 2;
+        if (bw > 64) return false;
+        g.np[hb] = nt / 2;
+        g.bw[hb] = bw;
+        g.w_off[hb] = off;
+        off += 4 * nt * TI * 4;
+        bwmax = std::max(bwmax, bw);
+    }
+    g.g_off = off;
+    g.x_off = off + t.nh * TI * 8;
+    g.tab_bytes = (g.x_off + 512 + 127) / 128 * 128;
+    g.stg_bytes = 4 * TC * bwmax * 8;
+    /* box coordinates (2 floats a bin) and bins in 32-bit ints */
+    const double xmax = (double)namps + FRONT + 7.0 * smax + 64;
+    double rmax = 0;
+    for (int h = 0; h < t.nh; h++) {
+        if (t.harm[h].rfloor0 < 0) return false;
+        rmax = std::max(rmax, (double)t.harm[h].rfloor0);
+    }
+    if (2.0 * xmax >= 2147483000.0 ||
+        2.0 * (rmax + (double)smax * (TC * (double)ncg + 2) + 64) >= 2147483000.0) return false;
+    g.nstg = MAX_STG;
+    while (g.nstg >= MIN_STG && layout(g, t.npad, t.kpad).total > max_smem) g.nstg--;
+    return g.nstg >= MIN_STG;
+}
+
+/* Tables, padded copy and tensor maps of the register-block kernel; false
+ * (with the session left on search_ws or the generic kernel) when the
+ * geometry does not fit or any step is refused. */
+static bool cols_load(GpuSession *S, const CsTables &t, long long total)
+{
+    using namespace cols;
+    const int nh = ladder_config(t, total);
+    if (!nh || S->prec64 || getenv("CS_B200_WS_KERNEL")) return false;
+    Geo &g = S->cx.g;
+    if (!cols_geometry(t, total, S->namps, S->max_smem, g)) return false;
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    S->cols_smem = layout(g, t.npad, t.kpad).total;
+    const size_t back = 7 * (size_t)g.shift[nh - 1] + 64;
+    const size_t nbins = FRONT + (size_t)S->namps + back;
+    if (dev_reserve((void **)&S->d_pad, &S->c_pad, nbins * sizeof(float2)) != cudaSuccess ||
+        dev_reserve((void **)&S->d_ctab, &S->c_ctab, (size_t)g.npb * g.tab_bytes) != cudaSuccess)
+        return false;
+    if (!S->d_cmaps &&
+        cudaMalloc((void **)&S->d_cmaps, sizeof(CUtensorMap) * wsk::MAX_NH) != cudaSuccess)
+        return false;
+    if (cudaMemsetAsync(S->d_pad, 0, FRONT * sizeof(float2), S->st) != cudaSuccess ||
+        cudaMemsetAsync(S->d_pad + FRONT + S->namps, 0, back * sizeof(float2), S->st) != cudaSuccess)
+        return false;
+    /* 8 rows, a column's shift apart; the inner extent keeps the last row
+     * inside the buffer, and the back pad keeps every bin inside the extent */
+    std::vector<CUtensorMap> maps((size_t)nh);
+    for (int h = 0; h < nh; h++) {
+        const cuuint64_t gdim[2] = {(cuuint64_t)(2 * (nbins - 7 * (size_t)g.shift[h])),
+                                    (cuuint64_t)TC};
+        const cuuint64_t gstr[1] = {(cuuint64_t)(8 * (size_t)g.shift[h])};
+        const cuuint32_t box[2] = {(cuuint32_t)(2 * g.bw[h / 4]), TC};
+        const cuuint32_t est[2] = {1, 1};
+        if (enc(&maps[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)S->d_pad, gdim, gstr, box,
+                est, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
+            CUDA_SUCCESS)
+            return false;
+    }
+    if (cudaMemcpyAsync(S->d_cmaps, maps.data(), maps.size() * sizeof(CUtensorMap),
+                        cudaMemcpyHostToDevice, S->st) != cudaSuccess)
+        return false;
+    table_kernel<<<dim3(g.npb, nh), 64, 0, S->st>>>(g, S->d_harm, S->d_rowtab, S->d_carry, S->d_W,
+                                                    S->d_A, t.q, t.pnum, t.m, S->d_ctab);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaFuncSetAttribute(cols_fn(nh), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             S->max_smem) != cudaSuccess ||
+        cudaStreamSynchronize(S->st) != cudaSuccess)       /* the maps' host copy goes */
+        return false;
+    S->cx.tab = S->d_ctab;
+    S->cx.maps = S->d_cmaps;
+    S->use_cols = nh;
+    return true;
+}
+
 static int ws_smem(int nh)
 {
     return nh == 60 ? wsk::smem_bytes<wsk::Cfg60>()
@@ -1377,9 +1536,12 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
     }
     S->use_tci = tci_load(S, t, total) ? 1 : 0;
     (void)cudaGetLastError();
+    S->use_cols = 0;
     S->use_tma = S->use_tci ? 0 : tma_config(t, total, S->namps, S->use_ws);
     if (S->use_tma && (tma_smem(S->use_tma) > S->max_smem || !tma_load(S, t, total)))
         S->use_tma = 0;
+    if (!S->use_tci && !S->use_tma) (void)cols_load(S, t, total);
+    (void)cudaGetLastError();
     {
         /* Start with room for 1 in 16 trials per slot; grown on overflow. */
         long long want = (total * t.nslot) / 16 + 4096;
@@ -1409,7 +1571,8 @@ static size_t session_bytes(const GpuSession *S)
     return S->c_amps + S->c_rowtab + S->c_W + S->c_A + S->c_carry + S->c_chunks + S->c_tiles +
            S->c_bimg + (size_t)S->cap * sizeof(CsRec) + sizeof(CsHarm) * CS_MAX_NH +
            S->c_bcs + S->c_scales + (size_t)S->cap64 * sizeof(CsRec64) + S->c_wtab +
-           S->c_cchunk + 2 * S->c_tc + (S->d_maps ? sizeof(CUtensorMap) * 2 * wsk::MAX_NH : 0) +
+           S->c_cchunk + 2 * S->c_tc + S->c_pad + S->c_ctab +
+           (S->d_cmaps ? sizeof(CUtensorMap) * wsk::MAX_NH : 0) + (S->d_maps ? sizeof(CUtensorMap) * 2 * wsk::MAX_NH : 0) +
            (S->d_Wt ? (size_t)wsk::MAX_NH * 4 * wsk::WT_STRIDE * sizeof(float4) : 0);
 }
 
@@ -1599,6 +1762,8 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
         if (S->use_tma)
             wsk::tma_prep_kernel<<<g, 256, 0, S->st>>>(d_amps, (int)S->namps, S->d_tc[0],
                                                        S->d_tc[1], S->d_amax);
+        else if (S->use_cols)
+            cols::pad_amax_kernel<<<g, 256, 0, S->st>>>(d_amps, (int)S->namps, S->d_pad, S->d_amax);
         else
             cs_amax_kernel<<<g, 256, 0, S->st>>>(d_amps, S->namps, S->d_amax);
     }
@@ -1645,6 +1810,13 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
         if (timed) cudaEventRecord(S->ev0, S->st);
         tci::interp_tc<<<grid1, tci::NTHREADS, tci::SMEM_BYTES, S->st>>>(ta);
         wsk::search_pre<wsk::Cfg60><<<grid, 512, ws_smem(60), S->st>>>(w);
+        if (timed) cudaEventRecord(S->ev1, S->st);
+        return cudaGetLastError();
+    }
+    if (S->use_cols) {
+        const int grid = std::min(S->cx.g.ntiles, S->nsm);
+        if (timed) cudaEventRecord(S->ev0, S->st);
+        cols_launch(S->use_cols, grid, S->cols_smem, S->st, ws_args(S, d_amps, threshold), S->cx);
         if (timed) cudaEventRecord(S->ev1, S->st);
         return cudaGetLastError();
     }
@@ -1841,9 +2013,12 @@ CS_EXPORT int cs_b200_session_info(const GpuSession *S, CsB200Info *info)
     info->npad = S->tab.npad;
     info->kpad = S->tab.kpad;
     info->smem_bytes = S->prec64 ? S->f64_smem : S->use_tma ? tma_smem(S->use_tma)
+                     : S->use_cols ? S->cols_smem
                      : S->use_ws ? ws_smem(S->use_ws) : smem_bytes(S->tab);
-    info->grid = S->use_tma ? std::min(S->tx.nitems, S->nsm) : std::min(S->tab.ntiles, S->nsm);
-    info->kernel = S->prec64 ? 2 : S->use_tci ? 4 : S->use_tma ? 3 : S->use_ws ? 1 : 0;
+    info->grid = S->use_tma ? std::min(S->tx.nitems, S->nsm)
+               : S->use_cols ? std::min(S->cx.g.ntiles, S->nsm) : std::min(S->tab.ntiles, S->nsm);
+    info->kernel = S->prec64 ? 2 : S->use_tci ? 4 : S->use_tma ? 3
+                 : S->use_cols || S->use_ws ? 1 : 0;
     info->total = S->total;
     info->rec_capacity = S->cap;
     return 0;
