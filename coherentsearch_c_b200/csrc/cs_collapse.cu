@@ -31,8 +31,9 @@
  * its own position in its slot plus, for every other slot, the number of
  * candidates there that come before it in (r, chunk, slot, j) order (a
  * binary search): the stable r order of the (chunk, slot, j) base order.
- * The metrics are FP32 values, so the metric sort uses 32-bit float keys.  The greedy pass runs in one
- * CTA: for each kept candidate, in metric order, the threads mark every later
+ * The
+ * metrics are FP32 values, so the metric sort uses 32-bit float keys.  The greedy
+ * pass runs in one CTA: for each kept candidate, in metric order, the threads mark every later
  * candidate it is related to; a candidate is kept when no earlier kept one
  * marked it, as in the host loop.  The FP64 expressions are the host's.
  */
@@ -190,16 +191,6 @@ __global__ void copy_count_kernel(const unsigned *src, unsigned *dst)
     *dst = *src;
 }
 
-/* descending-sort keys; entries past m sort after every real one */
-__global__ void gather_metric_kernel(const unsigned *list, const double *metric, unsigned n,
-                                     const unsigned *m, float *key, unsigned *pos)
-{
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    key[i] = i < *m ? (float)metric[list[i]] : -INFINITY;     /* FP32 values: exact */
-    pos[i] = i;
-}
-
 static __device__ bool related(double r1, double r2, int numharm, double tol)
 {
     const double lo = r1 < r2 ? r1 : r2;
@@ -213,95 +204,388 @@ static __device__ bool related(double r1, double r2, int numharm, double tol)
     return false;
 }
 
-/* remove_harmonics' greedy loop over the metric-ordered list (one CTA).
- * The walk is serial in the list, so with up to GREEDY_SMEM candidates the
- * positions' r values and the removal marks are staged in shared memory and
- * a step costs a shared read, not two dependent global loads; longer lists
- * walk global memory. */
-constexpr unsigned GREEDY_SMEM = 8192;
-__global__ void __launch_bounds__(1024) greedy_kernel(const unsigned *list, const unsigned *pos,
-                                                      const double *r, const unsigned *mp,
-                                                      int numharm, double tol,
-                                                      unsigned char *removed,
-                                                      unsigned char *keep_by_pos)
+/* ---- the last steps, in one CTA of FT threads ----
+ * remove_harmonics over a list of m candidates in frequency order: the
+ * stable descending metric order, the greedy walk over it, and the kept ones out
+ * in list order.  With up to CAP candidates everything is in shared memory; a
+ * step of the walk, which is serial in the list, then costs a shared read. */
+constexpr int FT = 1024;
+constexpr unsigned CAP = 4096;
+using MetricSort = cub::BlockRadixSort<uint32_t, FT, CAP / FT, uint16_t>;
+
+struct FinishShared {
+    double rs[CAP];                 /* r in metric order */
+    uint16_t pos[CAP];              /* list position of each */
+    unsigned char rm[CAP];          /* removed, in metric order */
+    unsigned char keep[CAP];        /* by list position */
+    unsigned warp_tot[32];
+    unsigned base;
+};
+
+/* keep[] for the m <= CAP candidates whose metric and r get(p) gives; stmp is
+ * the radix sort's storage.  Short lists are ranked by counting. */
+template <class Get>
+static __device__ void harmonics_keep(FinishShared &f, MetricSort::TempStorage &stmp, unsigned m,
+                                      int numharm, double tol, Get get)
 {
-    extern __shared__ double gsm[];               /* [GREEDY_SMEM] r, then the marks */
+    const unsigned tid = threadIdx.x;
+    if (m <= FT / 2) {
+        uint32_t *key = reinterpret_cast<uint32_t *>(&stmp);
+        double r = 0.0;
+        uint32_t k = 0;
+        if (tid < m) {
+            float mt;
+            get(tid, mt, r);
+            k = ordered_bits(mt + 0.0f);        /* -0 and 0 compare equal */
+            key[tid] = k;
+        }
+        __syncthreads();
+        if (tid < m) {
+            unsigned rank = 0;
+            for (unsigned i = 0; i < m; i++) {
+                const uint32_t o = key[i];
+                rank += o > k || (o == k && i < tid) ? 1u : 0u;
+            }
+            f.rs[rank] = r;
+            f.pos[rank] = (uint16_t)tid;
+            f.rm[rank] = 0;
+        }
+    } else {
+        uint32_t k[CAP / FT];
+        uint16_t v[CAP / FT];
+#pragma unroll
+        for (unsigned u = 0; u < CAP / FT; u++) {
+            const unsigned p = tid * (CAP / FT) + u;
+            float mt = 0.0f;
+            double r;
+            if (p < m) get(p, mt, r);
+            k[u] = p < m ? ~ordered_bits(mt + 0.0f) : 0xFFFFFFFFu;
+            v[u] = (uint16_t)p;
+        }
+        __syncthreads();
+        MetricSort(stmp).Sort(k, v);        /* stable: equal metrics stay in list order */
+        __syncthreads();
+#pragma unroll
+        for (unsigned u = 0; u < CAP / FT; u++) {
+            const unsigned q = tid * (CAP / FT) + u;
+            if (q < m) {
+                float mt;
+                double r;
+                get(v[u], mt, r);
+                f.rs[q] = r;
+                f.pos[q] = v[u];
+                f.rm[q] = 0;
+            }
+        }
+    }
+    __syncthreads();
+    for (unsigned i = 0; i < m; i++) {
+        if (f.rm[i]) continue;                  /* the same value in every thread */
+        const double ri = f.rs[i];
+        for (unsigned j = i + 1 + tid; j < m; j += FT)
+            if (!f.rm[j] && related(f.rs[j], ri, numharm, tol)) f.rm[j] = 1;
+        __syncthreads();
+    }
+    for (unsigned q = tid; q < m; q += FT) f.keep[f.pos[q]] = !f.rm[q];
+    __syncthreads();
+}
+
+/* The candidates p < m with keep(p), in order, to out; their number. */
+template <class Keep, class Put>
+static __device__ unsigned emit_kept(FinishShared &f, unsigned m, Keep keep, Put put)
+{
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) f.base = 0;
+    __syncthreads();
+    for (unsigned s = 0; s < m; s += FT) {
+        const unsigned i = s + threadIdx.x;
+        const bool k = i < m && keep(i);
+        const unsigned bal = __ballot_sync(0xffffffffu, k);
+        if (lane == 0) f.warp_tot[w] = __popc(bal);
+        __syncthreads();
+        unsigned off = f.base, all = 0;
+        for (unsigned q = 0; q < FT / 32; q++) {
+            if (q < w) off += f.warp_tot[q];
+            all += f.warp_tot[q];
+        }
+        if (k) put(i, off + __popc(bal & ((1u << lane) - 1u)));
+        __syncthreads();
+        if (threadIdx.x == 0) f.base += all;
+        __syncthreads();
+    }
+    return f.base;
+}
+
+static __device__ __forceinline__ Candidate make_cand(double r, double freq, double metric, int nharm)
+{
+    Candidate c;
+    c.freq = freq;
+    c.metric = metric;
+    c.r = r;
+    c.nharm = nharm;
+    c.ducy = NAN;
+    return c;
+}
+
+struct FinishSmem {
+    FinishShared f;
+    union {
+        MetricSort::TempStorage sort;
+        uint32_t keys[FT];
+    } t;
+};
+
+/* The last steps for a list in global memory.  Lists past CAP are ranked by
+ * counting and walked in global memory (the walk, not the ranking, is what they
+ * cost). */
+__global__ void __launch_bounds__(FT) finish_kernel(const unsigned *list, const unsigned *mp,
+                                                    int harm_remove, int numharm, double tol,
+                                                    const double *r, const double *freq,
+                                                    const double *metric, const int *nharm,
+                                                    unsigned *mpos, unsigned char *removed,
+                                                    unsigned char *keep, Candidate *out,
+                                                    unsigned *nout)
+{
+    extern __shared__ __align__(16) unsigned char fsm[];
+    FinishSmem &sm = *reinterpret_cast<FinishSmem *>(fsm);
     const unsigned m = *mp;
-    if (m <= GREEDY_SMEM) {
-        double *rs = gsm;
-        unsigned char *rm = reinterpret_cast<unsigned char *>(gsm + GREEDY_SMEM);
-        for (unsigned j = threadIdx.x; j < m; j += blockDim.x) {
-            rs[j] = r[list[pos[j]]];
-            rm[j] = 0;
+    const bool small = m <= CAP;
+    if (harm_remove && small) {
+        harmonics_keep(sm.f, sm.t.sort, m, numharm, tol, [&](unsigned p, float &mt, double &rr) {
+            const unsigned c = list[p];
+            mt = (float)metric[c];              /* FP32 values: exact */
+            rr = r[c];
+        });
+    } else if (harm_remove) {
+        for (unsigned p = threadIdx.x; p < m; p += FT) {
+            const float x = (float)metric[list[p]];
+            unsigned rank = 0;
+            for (unsigned i = 0; i < m; i++) {
+                const float y = (float)metric[list[i]];
+                rank += y > x || (y == x && i < p) ? 1u : 0u;
+            }
+            mpos[rank] = p;
+            removed[rank] = 0;
         }
         __syncthreads();
         for (unsigned i = 0; i < m; i++) {
-            if (rm[i]) continue;                    /* the same value in every thread */
-            const double ri = rs[i];
-            for (unsigned j = i + 1 + threadIdx.x; j < m; j += blockDim.x)
-                if (!rm[j] && related(rs[j], ri, numharm, tol)) rm[j] = 1;
+            if (removed[i]) continue;           /* the same value in every thread */
+            const double ri = r[list[mpos[i]]];
+            for (unsigned j = i + 1 + threadIdx.x; j < m; j += FT)
+                if (!removed[j] && related(r[list[mpos[j]]], ri, numharm, tol)) removed[j] = 1;
             __syncthreads();
         }
-        for (unsigned q = threadIdx.x; q < m; q += blockDim.x) keep_by_pos[pos[q]] = !rm[q];
-        return;
-    }
-    for (unsigned j = threadIdx.x; j < m; j += blockDim.x) removed[j] = 0;
-    __syncthreads();
-    for (unsigned i = 0; i < m; i++) {
-        if (removed[i]) continue;               /* the same value in every thread */
-        const double ri = r[list[pos[i]]];
-        for (unsigned j = i + 1 + threadIdx.x; j < m; j += blockDim.x)
-            if (!removed[j] && related(r[list[pos[j]]], ri, numharm, tol)) removed[j] = 1;
+        for (unsigned q = threadIdx.x; q < m; q += FT) keep[mpos[q]] = !removed[q];
         __syncthreads();
     }
-    for (unsigned q = threadIdx.x; q < m; q += blockDim.x) keep_by_pos[pos[q]] = !removed[q];
+    const unsigned n = emit_kept(
+        sm.f, m, [&](unsigned i) { return !harm_remove || (small ? sm.f.keep[i] : keep[i]); },
+        [&](unsigned i, unsigned o) {
+            const unsigned c = list[i];
+            out[o] = make_cand(r[c], freq[c], metric[c], nharm[c]);
+        });
+    if (threadIdx.x == 0) *nout = n;
 }
 
-__global__ void emit_kernel(const unsigned *list, const unsigned char *keep, const unsigned *mp,
-                            const double *r, const double *freq, const double *metric,
-                            const int *nharm, Candidate *out, unsigned *nout)
+/* ---- the whole collapse of up to CAP records in one CTA ----
+ * The same steps on shared memory: one launch where the long-list path has
+ * about twenty, none of which has work for more than a CTA then.  It reads the
+ * record count on the device, so it can be queued behind a search whose count
+ * the host does not know yet, and writes the list to pinned host memory: one
+ * wait in all.  (1 M points, 300 records: 33 us of kernel against 75 us of
+ * kernels, two waits and a copy; a whole pass 523 -> 428 us.) */
+template <unsigned IT>
+using SlotSort = cub::BlockRadixSort<uint32_t, FT, IT, uint16_t>;
+
+struct SmallArgs {
+    const CsRec *recs;
+    const unsigned *count;
+    const int *err;
+    unsigned cap;                   /* of the record buffer */
+    const CsChunk *chunks;
+    SlotInfo si;
+    int nslot;
+    uint32_t total;                 /* trials; nslot * total < 2^32 - 1 */
+    int end_bit;
+    double r_lo, lodr, nyq, T, thr;
+    int remove, harm_remove, numharm;
+    double drtol, tol;
+    Candidate *out;                 /* pinned, CAP */
+    unsigned *status;               /* pinned: records, error flag, list length, done */
+};
+
+struct SmallSmem {
+    double rr[CAP];                 /* r of each record */
+    float met[CAP];
+    int chunk[CAP];
+    unsigned char slot[CAP];
+    uint16_t list[CAP];             /* the best of each run */
+    unsigned cnt[CS_MAX_SLOT + 1], start[CS_MAX_SLOT + 1];
+    unsigned m;
+    union {
+        struct {
+            double v[CAP];          /* sort value (r or freq), slots in turn, rising in each */
+            uint16_t idx[CAP];      /* its record */
+            uint16_t ord[CAP];      /* records in (value, base) order */
+            union {
+                unsigned long long best[CAP];
+                SlotSort<1>::TempStorage sort1;
+                SlotSort<2>::TempStorage sort2;
+                SlotSort<4>::TempStorage sort4;
+            } u;
+            typename cub::BlockScan<unsigned, FT>::TempStorage scan;
+        } o;
+        FinishSmem fin;             /* once the list is made */
+    };
+};
+static_assert(sizeof(SmallSmem) <= 220 * 1024 && CAP == 4 * FT, "one CTA's shared memory");
+
+/* Harvest, order and remove_duplicates of n <= IT * FT records: sm.list, sm.m. */
+template <unsigned IT>
+static __device__ void small_list(SmallSmem &sm, const SmallArgs &a, unsigned n,
+                                  typename SlotSort<IT>::TempStorage &tmp)
 {
-    const unsigned m = *mp;
-    /* one CTA: an ordered compaction (m is a few thousand at most) */
-    __shared__ unsigned base;
-    __shared__ unsigned warp_tot[32];
-    if (threadIdx.x == 0) base = 0;
+    const unsigned tid = threadIdx.x;
+    if (tid <= CS_MAX_SLOT) sm.cnt[tid] = 0;
     __syncthreads();
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (unsigned s = 0; s < m; s += blockDim.x) {
-        const unsigned i = s + threadIdx.x;
-        const bool k = i < m && (keep == nullptr || keep[i]);
-        const unsigned bal = __ballot_sync(0xffffffffu, k);
-        if (lane == 0) warp_tot[w] = __popc(bal);
-        __syncthreads();
-        unsigned off = base;
-        for (unsigned q = 0; q < w; q++) off += warp_tot[q];
-        if (k) {
-            const unsigned c = list[i];
-            Candidate cd;
-            cd.freq = freq[c];
-            cd.metric = metric[c];
-            cd.r = r[c];
-            cd.nharm = nharm[c];
-            cd.ducy = NAN;
-            out[off + __popc(bal & ((1u << lane) - 1u))] = cd;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned t = 0;
-            for (unsigned q = 0; q < nw; q++) t += warp_tot[q];
-            base += t;
-        }
-        __syncthreads();
+    /* harvest */
+    uint32_t key[IT];
+    uint16_t val[IT];
+#pragma unroll
+    for (unsigned u = 0; u < IT; u++) {
+        const unsigned i = tid * IT + u;
+        key[u] = a.total * (uint32_t)a.nslot;       /* after every valid record */
+        val[u] = (uint16_t)i;
+        if (i >= n) continue;
+        const CsRec rc = a.recs[i];
+        if (!((double)rc.metric > a.thr) || rc.slot < 0 || rc.slot >= a.nslot) continue;
+        const long long i0 = a.chunks[rc.chunk].i0;
+        const double rstart = a.r_lo + (double)i0 * a.lodr;
+        const double rfreq = rstart + (double)rc.j * a.lodr;
+        const double kmul = (double)a.si.k[rc.slot];
+        const double rsel = kmul != 1.0 ? kmul * rfreq : rfreq;
+        if (rc.slot != 0 && !(rsel < a.nyq)) continue;
+        key[u] = (uint32_t)rc.slot * a.total + (uint32_t)(i0 + rc.j);
+        sm.rr[i] = rsel;
+        sm.met[i] = rc.metric;
+        sm.chunk[i] = rc.chunk;
+        sm.slot[i] = (unsigned char)rc.slot;
+        atomicAdd(&sm.cnt[rc.slot], 1u);
     }
-    if (threadIdx.x == 0) *nout = base;
+    __syncthreads();
+    SlotSort<IT>(tmp).Sort(key, val, 0, a.end_bit);
+    if (tid == 0) {
+        unsigned acc = 0;
+        for (int s = 0; s < a.nslot; s++) {
+            sm.start[s] = acc;
+            acc += sm.cnt[s];
+        }
+        sm.start[a.nslot] = acc;
+    }
+    __syncthreads();
+    const unsigned nv = sm.start[a.nslot];
+#pragma unroll
+    for (unsigned u = 0; u < IT; u++) {
+        const unsigned p = tid * IT + u;
+        if (p < nv) {
+            sm.o.idx[p] = val[u];
+            sm.o.v[p] = a.remove ? sm.rr[val[u]] : sm.rr[val[u]] / a.T;
+        }
+    }
+    __syncthreads();
+    /* merge the slots: a record's place in its own plus, for every other, the
+     * records there before it in (value, chunk, slot) order */
+    for (unsigned p = tid; p < nv; p += FT) {
+        const unsigned x = sm.o.idx[p];
+        const int s = sm.slot[x];
+        const double vx = sm.o.v[p];
+        unsigned rank = p - sm.start[s];
+        for (int t = 0; t < a.nslot; t++) {
+            if (t == s) continue;
+            const unsigned lo = sm.start[t], hi = sm.start[t + 1];
+            unsigned b = lo, e = hi;
+            while (b < e) {
+                const unsigned mid = (b + e) >> 1;
+                if (sm.o.v[mid] < vx) b = mid + 1;
+                else e = mid;
+            }
+            rank += b - lo;
+            if (b < hi && sm.o.v[b] == vx) {
+                const int cy = sm.chunk[sm.o.idx[b]], cx = sm.chunk[x];
+                if (cy < cx || (cy == cx && t < s)) rank++;
+            }
+        }
+        sm.o.ord[rank] = (uint16_t)x;
+    }
+    __syncthreads();
+    if (a.remove) {
+        for (unsigned i = tid; i < nv; i += FT) sm.o.u.best[i] = 0;
+        unsigned flag[IT], run[IT];
+#pragma unroll
+        for (unsigned u = 0; u < IT; u++) {
+            const unsigned i = tid * IT + u;
+            flag[u] = i < nv && (i == 0 || sm.rr[sm.o.ord[i]] - sm.rr[sm.o.ord[i - 1]] > a.drtol) ? 1u : 0u;
+        }
+        unsigned runs;
+        cub::BlockScan<unsigned, FT>(sm.o.scan).InclusiveSum(flag, run, runs);
+        __syncthreads();
+#pragma unroll
+        for (unsigned u = 0; u < IT; u++) {
+            const unsigned i = tid * IT + u;
+            if (i < nv)
+                atomicMax(&sm.o.u.best[run[u] - 1],
+                          ((unsigned long long)ordered_bits(sm.met[sm.o.ord[i]]) << 32) |
+                              (unsigned long long)(0xFFFFFFFFu - i));
+        }
+        __syncthreads();
+        for (unsigned q = tid; q < runs; q += FT)
+            sm.list[q] = sm.o.ord[0xFFFFFFFFu - (unsigned)(sm.o.u.best[q] & 0xFFFFFFFFull)];
+        if (tid == 0) sm.m = runs;
+    } else {
+        for (unsigned q = tid; q < nv; q += FT) sm.list[q] = sm.o.ord[q];
+        if (tid == 0) sm.m = nv;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(FT) collapse_small(const __grid_constant__ SmallArgs a)
+{
+    extern __shared__ __align__(16) unsigned char ssm[];
+    SmallSmem &sm = *reinterpret_cast<SmallSmem *>(ssm);
+    const unsigned tid = threadIdx.x;
+    const unsigned n = *a.count;
+    const int err = *a.err;
+    if (tid == 0) {
+        a.status[0] = n;
+        a.status[1] = (unsigned)err;
+        a.status[2] = 0;
+        a.status[3] = err == 0 && n <= a.cap && n <= CAP ? 1u : 0u;
+    }
+    if (err != 0 || n > a.cap || n > CAP || n == 0) return;
+    if (n <= FT) small_list<1>(sm, a, n, sm.o.u.sort1);
+    else if (n <= 2 * FT) small_list<2>(sm, a, n, sm.o.u.sort2);
+    else small_list<4>(sm, a, n, sm.o.u.sort4);
+    const unsigned m = sm.m;
+    if (a.harm_remove)
+        harmonics_keep(sm.fin.f, sm.fin.t.sort, m, a.numharm, a.tol,
+                       [&](unsigned p, float &mt, double &r) {
+                           mt = sm.met[sm.list[p]];
+                           r = sm.rr[sm.list[p]];
+                       });
+    const unsigned kept = emit_kept(
+        sm.fin.f, m, [&](unsigned i) { return !a.harm_remove || sm.fin.f.keep[i]; },
+        [&](unsigned i, unsigned o) {
+            const unsigned c = sm.list[i];
+            a.out[o] = make_cand(sm.rr[c], sm.rr[c] / a.T, (double)sm.met[c], a.si.Hk[sm.slot[c]]);
+        });
+    if (tid == 0) a.status[2] = kept;
 }
 
 }  // namespace cl
 
-/* The greedy kernel's shared-memory limit, raised once per device (the
+/* The one-CTA kernels' shared-memory limits, raised once per device (the
  * attribute belongs to the device that is current when it is set). */
-static cudaError_t greedy_prepare(size_t gsmem)
+static cudaError_t finish_prepare()
 {
     static std::atomic<unsigned long long> done{0};
     int dev = 0;
@@ -309,8 +593,12 @@ static cudaError_t greedy_prepare(size_t gsmem)
     if (e != cudaSuccess || dev < 0 || dev >= 64) return e;
     const unsigned long long bit = 1ULL << dev;
     if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-    e = cudaFuncSetAttribute((const void *)cl::greedy_kernel,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem);
+    e = cudaFuncSetAttribute((const void *)cl::finish_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(cl::FinishSmem));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void *)cl::collapse_small,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(cl::SmallSmem));
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_acq_rel);
     return e;
 }
@@ -325,8 +613,7 @@ struct CsCollapse {
     double *r, *freq, *metric;
     int *nharm;
     unsigned *flag, *runid, *list;
-    float *mkey[2];
-    unsigned *mpos[2];
+    unsigned *mpos;
     unsigned char *removed, *keep;
     Candidate *out;
     unsigned *counters;             /* device: nvalid, runs, kept; then per-slot counts
@@ -337,14 +624,20 @@ struct CsCollapse {
     void *temp;
     size_t temp_bytes;
     unsigned pending_n;             /* records of the enqueued collapse */
+    /* collapse_small's list and status (pinned), and whether it is queued */
+    Candidate *s_out;
+    unsigned *s_status;
+    bool small;
 };
 
 static void collapse_release_buffers(CsCollapse *w)
 {
     for (int b = 0; b < 2; b++) {
-        cudaFree(w->key[b]); cudaFree(w->idx[b]); cudaFree(w->mkey[b]); cudaFree(w->mpos[b]);
-        w->key[b] = nullptr; w->idx[b] = nullptr; w->mkey[b] = nullptr; w->mpos[b] = nullptr;
+        cudaFree(w->key[b]); cudaFree(w->idx[b]);
+        w->key[b] = nullptr; w->idx[b] = nullptr;
     }
+    cudaFree(w->mpos);
+    w->mpos = nullptr;
     cudaFree(w->bkey); cudaFree(w->slot_of); cudaFree(w->merged);
     w->bkey = nullptr; w->slot_of = nullptr; w->merged = nullptr;
     cudaFree(w->r); cudaFree(w->freq); cudaFree(w->metric); cudaFree(w->nharm);
@@ -370,9 +663,8 @@ static cudaError_t collapse_reserve(CsCollapse *w, size_t n)
     for (int b = 0; b < 2; b++) {
         AL(w->key[b], c * sizeof(uint64_t));
         AL(w->idx[b], c * sizeof(unsigned));
-        AL(w->mkey[b], c * sizeof(float));
-        AL(w->mpos[b], c * sizeof(unsigned));
     }
+    AL(w->mpos, c * sizeof(unsigned));
     AL(w->bkey, c * sizeof(uint64_t));
     AL(w->slot_of, c * sizeof(int));
     AL(w->merged, c * sizeof(unsigned));
@@ -390,16 +682,13 @@ static cudaError_t collapse_reserve(CsCollapse *w, size_t n)
 #undef AL
     if (e != cudaSuccess) return e;
     /* the largest CUB scratch any step needs at this capacity */
-    size_t t1 = 0, t2 = 0, t3 = 0;
+    size_t t1 = 0, t3 = 0;
     cub::DoubleBuffer<uint64_t> kb(w->key[0], w->key[1]);
     cub::DoubleBuffer<unsigned> ib(w->idx[0], w->idx[1]);
-    cub::DoubleBuffer<float> mb(w->mkey[0], w->mkey[1]);
-    cub::DoubleBuffer<unsigned> pb(w->mpos[0], w->mpos[1]);
     e = cub::DeviceRadixSort::SortPairs(nullptr, t1, kb, ib, (int)c);
-    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairsDescending(nullptr, t2, mb, pb, (int)c);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, t3, w->flag, w->runid, (int)c);
     if (e != cudaSuccess) return e;
-    w->temp_bytes = std::max(t1, std::max(t2, t3));
+    w->temp_bytes = std::max(t1, t3);
     e = cudaMalloc(&w->temp, w->temp_bytes);
     if (e == cudaSuccess) w->cap = c;
     return e;
@@ -409,10 +698,14 @@ CsCollapse *cs_collapse_new(void)
 {
     CsCollapse *w = (CsCollapse *)calloc(1, sizeof(CsCollapse));
     if (!w) return nullptr;
-    if (cudaMallocHost((void **)&w->h_counters, 4 * sizeof(unsigned)) != cudaSuccess) {
+    /* one pinned block: the short path's list, then its status and the counters */
+    if (cudaMallocHost((void **)&w->s_out, cl::CAP * sizeof(Candidate) + 8 * sizeof(unsigned)) !=
+        cudaSuccess) {
         free(w);
         return nullptr;
     }
+    w->s_status = (unsigned *)(w->s_out + cl::CAP);
+    w->h_counters = w->s_status + 4;
     return w;
 }
 
@@ -421,8 +714,8 @@ void cs_collapse_free(CsCollapse *w)
     if (!w) return;
     collapse_release_buffers(w);
     cudaFree(w->counters);
-    if (w->h_counters) cudaFreeHost(w->h_counters);
     if (w->h_out) cudaFreeHost(w->h_out);
+    if (w->s_out) cudaFreeHost(w->s_out);
     free(w);
 }
 
@@ -433,6 +726,64 @@ static int bit_length_u64(uint64_t v)
     return b;
 }
 
+int cs_collapse_small_enqueue(CsCollapse *w, const CsRec *recs, const unsigned *count,
+                              const int *err, unsigned cap, const CsChunk *chunks,
+                              const int *slot_k, const int *slot_Hk, int nslot, long long total,
+                              double r_lo, double lodr, double N, double T, double threshold,
+                              int remove, double dr_tol, int harm_remove, int numharm,
+                              double harm_tol, cudaStream_t st)
+{
+    if (!w || nslot < 1 || nslot > CS_MAX_SLOT || total < 1) return -1;
+    if ((unsigned long long)total * (unsigned long long)nslot >= 0xFFFFFFFFull) return 1;
+    cl::SmallArgs a;
+    memset(&a, 0, sizeof(a));
+    a.recs = recs;
+    a.count = count;
+    a.err = err;
+    a.cap = cap;
+    a.chunks = chunks;
+    for (int s = 0; s < nslot; s++) { a.si.k[s] = slot_k[s]; a.si.Hk[s] = slot_Hk[s]; }
+    a.nslot = nslot;
+    a.total = (uint32_t)total;
+    a.end_bit = bit_length_u64((uint64_t)total * (uint64_t)nslot);
+    a.r_lo = r_lo;
+    a.lodr = lodr;
+    a.nyq = N / 2.0;
+    a.T = T;
+    a.thr = threshold;
+    a.remove = remove;
+    a.harm_remove = harm_remove;
+    a.numharm = numharm;
+    a.drtol = dr_tol;
+    a.tol = harm_tol;
+    a.out = w->s_out;
+    a.status = w->s_status;
+    w->s_status[3] = 0;
+    cudaError_t e = finish_prepare();
+    if (e == cudaSuccess) {
+        cl::collapse_small<<<1, cl::FT, sizeof(cl::SmallSmem), st>>>(a);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        fprintf(stderr, "Error: candidate collapse on the GPU: %s\n", cudaGetErrorString(e));
+        return -1;
+    }
+    w->small = true;
+    return 0;
+}
+
+unsigned cs_collapse_small_cap(void)
+{
+    return cl::CAP;
+}
+
+int cs_collapse_small_status(const CsCollapse *w, unsigned *n, int *err)
+{
+    *n = w->s_status[0];
+    *err = (int)w->s_status[1];
+    return w->s_status[3] ? 1 : 0;
+}
+
 int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsChunk *chunks,
                         long long nchunks, const int *slot_k, const int *slot_Hk, int nslot,
                         int nprof, double r_lo, double lodr, double N, double T,
@@ -441,6 +792,7 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
 {
     if (!w || nslot < 1 || nslot > CS_MAX_SLOT || nprof < 1 || nchunks < 1) return -1;
     w->pending_n = n;
+    w->small = false;
     if (n == 0) return 0;
     cl::SlotInfo si;
     memset(&si, 0, sizeof(si));
@@ -449,7 +801,6 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
     const int end_bit = bit_length_u64((uint64_t)nchunks * (uint64_t)nslot * (uint64_t)nprof);
     size_t tb = 0;
     const unsigned *order = nullptr, *listp = nullptr;
-    const unsigned char *keep = nullptr;
     cudaError_t e = collapse_reserve(w, n);       /* allocates the counters on first use */
     if (e != cudaSuccess || !w->counters) {
         fprintf(stderr, "Error: candidate collapse on the GPU: %s\n", cudaGetErrorString(e));
@@ -508,32 +859,11 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
         }
         listp = order;
     }
-    if (harm_remove) {
-        if (e == cudaSuccess) {
-            cl::gather_metric_kernel<<<g, cl::NT, 0, st>>>(listp, w->metric, n, m, w->mkey[0],
-                                                           w->mpos[0]);
-            e = cudaGetLastError();
-        }
-        cub::DoubleBuffer<float> mb(w->mkey[0], w->mkey[1]);
-        cub::DoubleBuffer<unsigned> pb(w->mpos[0], w->mpos[1]);
-        if (e == cudaSuccess) {
-            tb = w->temp_bytes;
-            e = cub::DeviceRadixSort::SortPairsDescending(w->temp, tb, mb, pb, (int)n, 0, 32, st);
-        }
-        if (e == cudaSuccess) {
-            const size_t gsmem = cl::GREEDY_SMEM * (sizeof(double) + 1);
-            e = greedy_prepare(gsmem);
-            if (e == cudaSuccess) {
-                cl::greedy_kernel<<<1, 1024, gsmem, st>>>(listp, pb.Current(), w->r, m, numharm,
-                                                          harm_tol, w->removed, w->keep);
-                e = cudaGetLastError();
-            }
-        }
-        keep = w->keep;
-    }
+    if (e == cudaSuccess) e = finish_prepare();
     if (e == cudaSuccess) {
-        cl::emit_kernel<<<1, 1024, 0, st>>>(listp, keep, m, w->r, w->freq, w->metric,
-                                            w->nharm, w->out, nout);
+        cl::finish_kernel<<<1, cl::FT, sizeof(cl::FinishSmem), st>>>(
+            listp, m, harm_remove, numharm, harm_tol, w->r, w->freq, w->metric, w->nharm, w->mpos,
+            w->removed, w->keep, w->out, nout);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
@@ -550,9 +880,21 @@ int cs_collapse_finish(CsCollapse *w, cudaStream_t st, CandidateList *out)
 {
     candlist_init(out);
     if (!w) return -1;
-    if (w->pending_n == 0) return 0;
+    if (!w->small && w->pending_n == 0) return 0;
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) goto fail;
+    if (w->small) {
+        const unsigned nout = w->s_status[2];
+        w->small = false;
+        if (nout) {
+            out->v = (Candidate *)malloc((size_t)nout * sizeof(Candidate));
+            if (!out->v) return -1;
+            memcpy(out->v, w->s_out, (size_t)nout * sizeof(Candidate));
+            out->n = nout;
+            out->cap = nout;
+        }
+        return 0;
+    }
     {
         const unsigned nout = w->h_counters[2];
         if (nout > w->h_out_cap) {

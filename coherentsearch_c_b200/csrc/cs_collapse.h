@@ -20,6 +20,22 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
                         double threshold, int remove, double dr_tol, int harm_remove,
                         int numharm, double harm_tol, cudaStream_t st);
 
+/* The same for a search whose record count is still on the device (count, err:
+ * the search's counter and error flag; cap: the record buffer's capacity; total:
+ * trials), in one launch that only works on up to cs_collapse_small_cap()
+ * records.  After a wait on `st`, cs_collapse_small_status gives the count and
+ * the error flag, and 1 when the list is ready (cs_collapse_finish hands it
+ * over), 0 when the records have to go through cs_collapse_enqueue.  Returns 0, 1
+ * when the geometry does not fit (nothing queued), or -1. */
+int cs_collapse_small_enqueue(CsCollapse *w, const CsRec *recs, const unsigned *count,
+                              const int *err, unsigned cap, const CsChunk *chunks,
+                              const int *slot_k, const int *slot_Hk, int nslot, long long total,
+                              double r_lo, double lodr, double N, double T, double threshold,
+                              int remove, double dr_tol, int harm_remove, int numharm,
+                              double harm_tol, cudaStream_t st);
+unsigned cs_collapse_small_cap(void);
+int cs_collapse_small_status(const CsCollapse *w, unsigned *n, int *err);
+
 /* Wait for the enqueued collapse and copy its list to host memory (out;
  * the caller frees it with candlist_free).  0 or -1. */
 int cs_collapse_finish(CsCollapse *w, cudaStream_t st, CandidateList *out);

@@ -671,7 +671,7 @@ struct GpuSession {
     bool img_ok;
     int img_nh, img_nslot, img_npad, img_kpad;
     CsSlot img_slot[CS_MAX_SLOT];
-    unsigned *d_amax;      /* [2] */
+    unsigned *d_amax;      /* [2]; d_count and d_err follow in the same buffer */
     unsigned *d_count;     /* [1] */
     int *d_err;            /* [1] */
     CsRec *d_recs;
@@ -704,10 +704,10 @@ struct GpuSession {
     int use_cols;
     cols::XArgs cx;
     int cols_smem;
-    float2 *d_pad;         /* padded spectrum copy */
-    unsigned char *d_ctab;
-    CUtensorMap *d_cmaps;  /* [nh] */
-    size_t c_pad, c_ctab;
+    unsigned char *d_cols; /* tensor maps [nh], tables, padded spectrum copy */
+    size_t c_cols;
+    float2 *d_pad;         /* the copy, in d_cols */
+    CUtensorMap *h_cmaps;  /* [MAX_NH], 64-byte aligned */
     /* interpolation as tensor-core GEMMs (tci::interp_tc), then search_pre */
     int use_tci;
     tci::Band *d_tci_bands;
@@ -789,8 +789,6 @@ static void session_release(GpuSession *S)
     cudaFree(S->d_tiles);
     cudaFree(S->d_bimg);
     cudaFree(S->d_amax);
-    cudaFree(S->d_count);
-    cudaFree(S->d_err);
     cudaFree(S->d_recs);
     cudaFree(S->d_Wt);
     cudaFree(S->d_AC);
@@ -800,9 +798,8 @@ static void session_release(GpuSession *S)
     cudaFree(S->d_maps);
     cudaFree(S->d_tc[0]);
     cudaFree(S->d_tc[1]);
-    cudaFree(S->d_pad);
-    cudaFree(S->d_ctab);
-    cudaFree(S->d_cmaps);
+    cudaFree(S->d_cols);
+    free(S->h_cmaps);
     cudaFree(S->d_tci_bands);
     cudaFree(S->d_tci_bimg);
     cudaFree(S->d_tci_hbase);
@@ -1284,42 +1281,43 @@ static bool cols_load(GpuSession *S, const CsTables &t, long long total)
     S->cols_smem = layout(g, t.npad, t.kpad).total;
     const size_t back = 7 * (size_t)g.shift[nh - 1] + 64;
     const size_t nbins = FRONT + (size_t)S->namps + back;
-    if (dev_reserve((void **)&S->d_pad, &S->c_pad, nbins * sizeof(float2)) != cudaSuccess ||
-        dev_reserve((void **)&S->d_ctab, &S->c_ctab, (size_t)g.npb * g.tab_bytes) != cudaSuccess)
+    const size_t tab_off = sizeof(CUtensorMap) * wsk::MAX_NH;
+    const size_t pad_off = tab_off + (size_t)g.npb * g.tab_bytes;      /* multiples of 128 */
+    if (dev_reserve((void **)&S->d_cols, &S->c_cols, pad_off + nbins * sizeof(float2)) != cudaSuccess)
         return false;
-    if (!S->d_cmaps &&
-        cudaMalloc((void **)&S->d_cmaps, sizeof(CUtensorMap) * wsk::MAX_NH) != cudaSuccess)
-        return false;
+    S->d_pad = (float2 *)(S->d_cols + pad_off);
+    if (!S->h_cmaps)
+        S->h_cmaps = (CUtensorMap *)aligned_alloc(64, sizeof(CUtensorMap) * wsk::MAX_NH);
+    if (!S->h_cmaps) return false;
     if (cudaMemsetAsync(S->d_pad, 0, FRONT * sizeof(float2), S->st) != cudaSuccess ||
         cudaMemsetAsync(S->d_pad + FRONT + S->namps, 0, back * sizeof(float2), S->st) != cudaSuccess)
         return false;
     /* 8 rows, a column's shift apart; the inner extent keeps the last row
      * inside the buffer, and the back pad keeps every bin inside the extent */
-    std::vector<CUtensorMap> maps((size_t)nh);
     for (int h = 0; h < nh; h++) {
         const cuuint64_t gdim[2] = {(cuuint64_t)(2 * (nbins - 7 * (size_t)g.shift[h])),
                                     (cuuint64_t)TC};
         const cuuint64_t gstr[1] = {(cuuint64_t)(8 * (size_t)g.shift[h])};
         const cuuint32_t box[2] = {(cuuint32_t)(2 * g.bw[h / 4]), TC};
         const cuuint32_t est[2] = {1, 1};
-        if (enc(&maps[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)S->d_pad, gdim, gstr, box,
+        if (enc(&S->h_cmaps[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)S->d_pad, gdim, gstr, box,
                 est, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
             CUDA_SUCCESS)
             return false;
     }
-    if (cudaMemcpyAsync(S->d_cmaps, maps.data(), maps.size() * sizeof(CUtensorMap),
-                        cudaMemcpyHostToDevice, S->st) != cudaSuccess)
+    /* the caller waits for the stream before the session is used */
+    if (cudaMemcpyAsync(S->d_cols, S->h_cmaps, sizeof(CUtensorMap) * nh, cudaMemcpyHostToDevice,
+                        S->st) != cudaSuccess)
         return false;
     table_kernel<<<dim3(g.npb, nh), 64, 0, S->st>>>(g, S->d_harm, S->d_rowtab, S->d_carry, S->d_W,
-                                                    S->d_A, t.q, t.pnum, t.m, S->d_ctab);
+                                                    S->d_A, t.q, t.pnum, t.m, S->d_cols + tab_off);
     if (cudaGetLastError() != cudaSuccess ||
         cudaFuncSetAttribute(cols_fn(nh), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             S->max_smem) != cudaSuccess ||
-        cudaStreamSynchronize(S->st) != cudaSuccess)       /* the maps' host copy goes */
+                             S->max_smem) != cudaSuccess)
         return false;
-    S->cx.tab = S->d_ctab;
-    S->cx.maps = S->d_cmaps;
+    S->cx.tab = S->d_cols + tab_off;
+    S->cx.maps = S->d_cols;
     S->use_cols = nh;
     return true;
 }
@@ -1571,8 +1569,7 @@ static size_t session_bytes(const GpuSession *S)
     return S->c_amps + S->c_rowtab + S->c_W + S->c_A + S->c_carry + S->c_chunks + S->c_tiles +
            S->c_bimg + (size_t)S->cap * sizeof(CsRec) + sizeof(CsHarm) * CS_MAX_NH +
            S->c_bcs + S->c_scales + (size_t)S->cap64 * sizeof(CsRec64) + S->c_wtab +
-           S->c_cchunk + 2 * S->c_tc + S->c_pad + S->c_ctab +
-           (S->d_cmaps ? sizeof(CUtensorMap) * wsk::MAX_NH : 0) + (S->d_maps ? sizeof(CUtensorMap) * 2 * wsk::MAX_NH : 0) +
+           S->c_cchunk + 2 * S->c_tc + S->c_cols + (S->d_maps ? sizeof(CUtensorMap) * 2 * wsk::MAX_NH : 0) +
            (S->d_Wt ? (size_t)wsk::MAX_NH * 4 * wsk::WT_STRIDE * sizeof(float4) : 0);
 }
 
@@ -1595,9 +1592,9 @@ static GpuSession *session_new(int device)
     CK(cudaEventCreate(&S->ev1));
     CK(cudaEventCreateWithFlags(&S->ev_in, cudaEventDisableTiming));
     CK(cudaMalloc((void **)&S->d_harm, sizeof(CsHarm) * CS_MAX_NH));
-    CK(cudaMalloc((void **)&S->d_amax, 2 * sizeof(unsigned)));
-    CK(cudaMalloc((void **)&S->d_count, sizeof(unsigned)));
-    CK(cudaMalloc((void **)&S->d_err, sizeof(int)));
+    CK(cudaMalloc((void **)&S->d_amax, 4 * sizeof(unsigned)));
+    S->d_count = S->d_amax + 2;
+    S->d_err = (int *)(S->d_amax + 3);
     CK(cudaMallocHost((void **)&S->h_count, 4 * sizeof(unsigned)));
     return S;
 fail:
@@ -1754,9 +1751,8 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
                                   bool timed)
 {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(S->d_amax, 0, 2 * sizeof(unsigned), S->st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(S->d_count, 0, sizeof(unsigned), S->st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(S->d_err, 0, sizeof(int), S->st)) != cudaSuccess) return e;
+    /* the spectrum maximum, the record count and the error flag */
+    if ((e = cudaMemsetAsync(S->d_amax, 0, 4 * sizeof(unsigned), S->st)) != cudaSuccess) return e;
     if (S->namps > 0) {
         int g = (int)std::min<long long>((S->namps + 255) / 256, (long long)S->nsm * 8);
         if (S->use_tma)
@@ -1888,10 +1884,8 @@ static int collect(GpuSession *S, double threshold, CandidateList *out, int *nee
 {
     *need_rerun = 0;
     cudaError_t e;
-    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(S->h_count + 1, S->d_err, sizeof(int), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                             S->st)) != cudaSuccess ||       /* the count and the error flag */
         (e = cudaStreamSynchronize(S->st)) != cudaSuccess) {
         fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
         return -1;
@@ -2065,6 +2059,21 @@ CS_EXPORT int cs_b200_session_collect(GpuSession *S, double threshold, Candidate
     return rerun ? 1 : 0;
 }
 
+/* Queue the one-launch collapse behind the search; 0, 1 (does not fit) or -1. */
+static int collapse_small(GpuSession *S, double threshold, int remove, double dr_tol,
+                          int harm_remove, int numharm, double harm_tol)
+{
+    int k[CS_MAX_SLOT], Hk[CS_MAX_SLOT];
+    for (int i = 0; i < S->tab.nslot; i++) {
+        k[i] = S->tab.slot[i].k;
+        Hk[i] = S->tab.slot[i].Hk;
+    }
+    return cs_collapse_small_enqueue(S->coll, S->d_recs, S->d_count, S->d_err, S->cap, S->d_chunks,
+                                     k, Hk, S->tab.nslot, S->total, S->r_lo, S->lodr,
+                                     (double)S->N, S->T, threshold, remove, dr_tol, harm_remove,
+                                     numharm, harm_tol, S->st);
+}
+
 CS_EXPORT int cs_b200_session_collapse_enqueue(GpuSession *S, double threshold, int remove,
                                                double dr_tol, int harm_remove, int numharm,
                                                double harm_tol)
@@ -2076,10 +2085,8 @@ CS_EXPORT int cs_b200_session_collapse_enqueue(GpuSession *S, double threshold, 
         return -1;
     }
     cudaError_t e;
-    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(S->h_count + 1, S->d_err, sizeof(int), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                             S->st)) != cudaSuccess ||       /* the count and the error flag */
         (e = cudaStreamSynchronize(S->st)) != cudaSuccess) {
         fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
         return -1;
@@ -2094,6 +2101,10 @@ CS_EXPORT int cs_b200_session_collapse_enqueue(GpuSession *S, double threshold, 
         return 1;
     }
     if (!S->coll && !(S->coll = cs_collapse_new())) return -1;
+    if (n > 0 && n <= cs_collapse_small_cap()) {
+        const int rc = collapse_small(S, threshold, remove, dr_tol, harm_remove, numharm, harm_tol);
+        if (rc <= 0) return rc;
+    }
     int k[CS_MAX_SLOT], Hk[CS_MAX_SLOT];
     for (int i = 0; i < S->tab.nslot; i++) {
         k[i] = S->tab.slot[i].k;
@@ -2121,6 +2132,24 @@ CS_EXPORT int cs_b200_session_collect_collapsed(GpuSession *S, double threshold,
 {
     if (!S || !out) return -1;
     candlist_init(out);
+    /* short record lists, the usual ones: one launch behind the search, which
+     * finds the count itself, and one wait */
+    if (!S->prec64 && S->total > 0) {
+        if (!S->coll && !(S->coll = cs_collapse_new())) return -1;
+        const int rs = collapse_small(S, threshold, remove, dr_tol, harm_remove, numharm, harm_tol);
+        if (rs < 0) return -1;
+        if (rs == 0) {
+            const cudaError_t e = cudaStreamSynchronize(S->st);
+            if (e != cudaSuccess) {
+                fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
+                return -1;
+            }
+            unsigned n;
+            int err;
+            if (cs_collapse_small_status(S->coll, &n, &err))
+                return cs_b200_session_collapse_wait(S, out, kernel_ms);
+        }
+    }
     const int rc = cs_b200_session_collapse_enqueue(S, threshold, remove, dr_tol, harm_remove,
                                                     numharm, harm_tol);
     if (rc != 0) return rc;
