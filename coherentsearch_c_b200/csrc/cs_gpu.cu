@@ -721,8 +721,12 @@ struct GpuSession {
     /* FP64 search (p->precision == CS_PREC_F64) */
     int prec64;
     f64k::Extra fx;
+    f64k::Wide fw;
+    int f64_wide;          /* search_f64_wide fits */
     int f64_smem;
     double *d_bcs, *d_scales;
+    float4 *d_wt64;        /* search_f64_wide's weights */
+    size_t c_wt64;
     CsRec64 *d_recs64;
     unsigned cap64;
     CsRec64 *h_recs64;     /* pinned record staging */
@@ -805,6 +809,7 @@ static void session_release(GpuSession *S)
     cudaFree(S->d_tci_hbase);
     cudaFree(S->d_X);
     cudaFree(S->d_bcs);
+    cudaFree(S->d_wt64);
     cudaFree(S->d_scales);
     cudaFree(S->d_recs64);
     if (S->h_recs64) cudaFreeHost(S->h_recs64);
@@ -1488,6 +1493,19 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
                             "%d allows %d\n", S->f64_smem, S->device, S->max_smem);
             return -1;
         }
+        {
+            f64k::Wide &w = S->fw;
+            memset(&w, 0, sizeof(w));
+            w.bstr = f64k::table_stride(x.ucols);
+            w.kp = (t.nh + 3) / 4 * 4;
+            for (int q = 0; q < t.nslot; q++) w.nwmax = std::max(w.nwmax, t.slot[q].nw);
+            f64k::deal(w, t.nslot, t.slot);
+            w.reg_pr = std::max(f64k::TT * x.prs, f64k::NW * w.nwmax * f64k::TT);
+            const int wide = f64k::wide_smem(w, x.ps_total);
+            S->f64_wide = wide + (int)sizeof(CsHarm) * CS_MAX_NH <= S->max_smem &&
+                          !getenv("CS_B200_GENERIC_KERNEL");
+            if (S->f64_wide) S->f64_smem = wide;
+        }
         CK(dev_reserve((void **)&S->d_bcs, &S->c_bcs, bcs.size() * sizeof(double)));
         CK(cudaMemcpyAsync(S->d_bcs, bcs.data(), bcs.size() * sizeof(double),
                            cudaMemcpyHostToDevice, S->st));
@@ -1495,6 +1513,13 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
         CK(dev_reserve((void **)&S->d_scales, &S->c_scales, nsc * sizeof(double)));
         CK(cudaMemcpyAsync(S->d_scales, t.invsw64, nsc * sizeof(double), cudaMemcpyHostToDevice,
                            S->st));
+        if (S->f64_wide && t.m == 16) {
+            CK(dev_reserve((void **)&S->d_wt64, &S->c_wt64, (size_t)t.nrows * t.m * sizeof(float)));
+            CK(cudaMemcpyAsync(S->d_wt64, t.Wt, (size_t)t.nrows * t.m * sizeof(float),
+                               cudaMemcpyHostToDevice, S->st));
+            x.wt = S->d_wt64;
+            memcpy(x.wt_off, t.wt_off, sizeof(int) * t.nh);
+        }
         x.bcs = S->d_bcs;
         x.scales = S->d_scales;
         long long want = (total * t.nslot) / 16 + 4096;
@@ -1504,6 +1529,8 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
         x.recs = S->d_recs64;
         CK(set_smem_cap((const void *)f64k::search_f64<16>, S->max_smem));
         CK(set_smem_cap((const void *)f64k::search_f64<0>, S->max_smem));
+        CK(set_smem_cap((const void *)f64k::search_f64_wide<16>, S->max_smem));
+        CK(set_smem_cap((const void *)f64k::search_f64_wide<0>, S->max_smem));
     }
     S->use_ws = S->prec64 ? 0 : ws_config(t, total);
     if (S->use_ws && (S->namps >= 2147483000LL || ws_smem(S->use_ws) > S->max_smem))
@@ -1568,7 +1595,7 @@ static size_t session_bytes(const GpuSession *S)
 {
     return S->c_amps + S->c_rowtab + S->c_W + S->c_A + S->c_carry + S->c_chunks + S->c_tiles +
            S->c_bimg + (size_t)S->cap * sizeof(CsRec) + sizeof(CsHarm) * CS_MAX_NH +
-           S->c_bcs + S->c_scales + (size_t)S->cap64 * sizeof(CsRec64) + S->c_wtab +
+           S->c_bcs + S->c_scales + S->c_wt64 + (size_t)S->cap64 * sizeof(CsRec64) + S->c_wtab +
            S->c_cchunk + 2 * S->c_tc + S->c_cols + (S->d_maps ? sizeof(CUtensorMap) * 2 * wsk::MAX_NH : 0) +
            (S->d_Wt ? (size_t)wsk::MAX_NH * 4 * wsk::WT_STRIDE * sizeof(float4) : 0);
 }
@@ -1772,7 +1799,11 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
         const int nsub = S->tab.ntiles * (CS_TILE_M / f64k::TT);
         const int grid = std::min(nsub, S->nsm);
         if (timed) cudaEventRecord(S->ev0, S->st);
-        if (S->tab.m == 16)
+        if (S->f64_wide && S->tab.m == 16)
+            f64k::search_f64_wide<16><<<grid, f64k::WNT, S->f64_smem, S->st>>>(a64, x, S->fw);
+        else if (S->f64_wide)
+            f64k::search_f64_wide<0><<<grid, f64k::WNT, S->f64_smem, S->st>>>(a64, x, S->fw);
+        else if (S->tab.m == 16)
             f64k::search_f64<16><<<grid, f64k::NT, S->f64_smem, S->st>>>(a64, x);
         else
             f64k::search_f64<0><<<grid, f64k::NT, S->f64_smem, S->st>>>(a64, x);
