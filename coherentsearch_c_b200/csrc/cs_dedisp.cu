@@ -199,6 +199,7 @@ struct SubArgs {
     long long sfill;          /* samples written per subband */
     uint32_t *sub;            /* S: [nsub][sstride] words (samples w, w + DM_P) */
     long long sstride;
+    const uint8_t *need;      /* clipped runs: tiles some DM item reads (null: all) */
     /* clipped runs (dd_subband_clip) */
     const uint8_t *flags;     /* [nflags] 1: spectrum replaced */
     long long nflags;
@@ -253,6 +254,7 @@ static __device__ __forceinline__ void sb_stage(const SubArgs &a, unsigned char 
 __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8(const SubArgs a)
 {
     extern __shared__ __align__(16) unsigned char sm[];
+    if (a.need && !a.need[blockIdx.y]) return;
     const int s0 = blockIdx.x * a.slab;                   /* first subband */
     const int nslab = min(a.slab, a.nsub - s0);
     const int sc = nslab * a.cps;                         /* channels staged */
@@ -283,6 +285,52 @@ __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8(const SubArgs a)
     }
 }
 
+/* The same for slabs of 256 channels in whole subbands of CPS (rows of 260
+ * bytes): a warp keeps one subband, its channels' offsets in registers and the
+ * row stride in the instructions, so that a channel of 32 samples costs one
+ * shared load and half an addition (the general kernel also reads the offset and
+ * adds it), and writes both halves of a word at once where it has them.  Bound by
+ * the shared loads and the staging; 500 k spectra of 1024 channels: 253 us in
+ * the general kernel, MEASURED_SB here, 79 us for the bytes read. */
+constexpr int SB_RS = 260;
+template <int CPS>
+__global__ void __launch_bounds__(SB_THREADS) dd_subband_u8_256(const SubArgs a)
+{
+    extern __shared__ __align__(16) unsigned char sm[];
+    if (a.need && !a.need[blockIdx.y]) return;
+    const int s0 = blockIdx.x * a.slab;
+    const long long T0 = (long long)blockIdx.y * SB_TT;
+    sb_stage(a, sm, s0, a.slab * CPS, T0);
+    const int *coff = reinterpret_cast<const int *>(sm + a.table_off);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NG = SB_TT / 32, HG = DM_P / 32;
+    static_assert(NG == 2 * HG, "a tile is both halves of its first words");
+    for (int sl = warp; sl < a.slab; sl += SB_THREADS / 32) {
+        const unsigned char *base[CPS];
+#pragma unroll
+        for (int k = 0; k < CPS; k++) base[k] = sm + lane * SB_RS + coff[sl * CPS + k];
+        uint32_t acc[NG];
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            acc[g] = 0;
+#pragma unroll
+            for (int k = 0; k < CPS; k += 2)
+                acc[g] += (uint32_t)base[k][g * 32 * SB_RS] + (uint32_t)base[k + 1][g * 32 * SB_RS];
+            if (T0 + g * 32 + lane >= a.nvalid) acc[g] = 0;
+        }
+        uint32_t *row = a.sub + (long long)(s0 + sl) * a.sstride;
+        uint16_t *row16 = reinterpret_cast<uint16_t *>(row);
+#pragma unroll
+        for (int g = 0; g < HG; g++) {
+            const long long T = T0 + g * 32 + lane;
+            if (T + DM_P < a.sfill) row[T] = acc[g] | (acc[g + HG] << 16);
+            else if (T < a.sfill) row16[2 * T] = (uint16_t)acc[g];
+            if (T >= DM_P && T < a.sfill) row16[2 * (T - DM_P) + 1] = (uint16_t)acc[g];
+            if (T + DM_P < a.sfill) row16[2 * (T + DM_P)] = (uint16_t)acc[g + HG];
+        }
+    }
+}
+
 /* The subband stage of a clipped run: spectra flagged by the clip decisions
  * take their block's channel levels (floats), so the sums are evaluated as
  * the reference does (dispersion.c:245-264): in FP32, from 0.0f, adding the
@@ -290,6 +338,7 @@ __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8(const SubArgs a)
 __global__ void __launch_bounds__(SB_THREADS) dd_subband_clip(const SubArgs a)
 {
     extern __shared__ __align__(16) unsigned char sm[];
+    if (a.need && !a.need[blockIdx.y]) return;
     const int s0 = blockIdx.x * a.slab;
     const int nslab = min(a.slab, a.nsub - s0);
     const int sc = nslab * a.cps;
@@ -351,11 +400,25 @@ struct DmArgs {
     int code_word, zero_word; /* word offsets in a stage */
     int stage_words, nstage;
     long long nitems;         /* tiles x groups */
+    const int *list, *count;  /* clipped runs: the items to do (null: all) */
     long long nout;
     float *out;
     long long ostride;
     int *err;                 /* set when a wait gave up */
 };
+
+/* The i-th item of a run and the number of items: all of them, or a list's. */
+template <class A>
+static __device__ __forceinline__ long long item_at(const A &a, long long i)
+{
+    return a.list ? (long long)__ldg(a.list + i) : i;
+}
+
+template <class A>
+static __device__ __forceinline__ long long item_count(const A &a)
+{
+    return a.list ? (long long)__ldg(a.count) : a.nitems;
+}
 
 /* The integer DM stage, warp-specialised over a ring of nstage shared
  * buffers.  Work item = (tile of DM_TILE samples, group of G consecutive
@@ -391,13 +454,14 @@ __global__ void __launch_bounds__(DM_THREADS, 1) dd_dms_u16(const DmArgs a)
         for (int i = threadIdx.x; i < DM_P; i += blockDim.x)
             smw[(size_t)st * a.stage_words + a.zero_word + i] = 0;
     __syncthreads();
-    const long long grid = gridDim.x;
+    const long long grid = gridDim.x, nitems = item_count(a);
 
     if (warp == DM_NCW) {
         /* ------------------------------ copy warp ------------------------------ */
         long long k = 0;
         bool ok = true;
-        for (long long item = blockIdx.x; item < a.nitems; item += grid, k++) {
+        for (long long i = blockIdx.x; i < nitems; i += grid, k++) {
+            const long long item = item_at(a, i);
             const int st = (int)(k % NS);
             const uint32_t ph = (uint32_t)(k / NS) & 1u;
             if (k >= NS) ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * st, ph ^ 1u));
@@ -427,7 +491,10 @@ __global__ void __launch_bounds__(DM_THREADS, 1) dd_dms_u16(const DmArgs a)
 
     /* ---------------------------- summing warps ---------------------------- */
     long long k = 0;
-    for (long long item = blockIdx.x; item < a.nitems; item += grid, k++) {
+    long long ahead = blockIdx.x < nitems ? item_at(a, blockIdx.x) : 0;
+    for (long long i = blockIdx.x; i < nitems; i += grid, k++) {
+        const long long item = ahead;
+        if (i + grid < nitems) ahead = item_at(a, i + grid);
         const int st = (int)(k % NS);
         const uint32_t ph = (uint32_t)(k / NS) & 1u;
         if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, ph))) {
@@ -676,6 +743,7 @@ struct FdArgs {
     const int *gbytes;        /* [ngroups]: bytes of the group's windows */
     int code_bytes, code_word, stage_words, nstage;
     long long nitems;
+    const int *list, *count;
     long long nout;
     float *out;
     long long ostride;
@@ -697,13 +765,14 @@ __global__ void __launch_bounds__(FD_THREADS, 1) dd_dms_f32_ws(const FdArgs a)
         mbar_fence_init();
     }
     __syncthreads();
-    const long long grid = gridDim.x;
+    const long long grid = gridDim.x, nitems = item_count(a);
 
     if (warp == FD_NCW) {
         /* ------------------------------ copy warp ------------------------------ */
         long long k = 0;
         bool ok = true;
-        for (long long item = blockIdx.x; item < a.nitems; item += grid, k++) {
+        for (long long i = blockIdx.x; i < nitems; i += grid, k++) {
+            const long long item = item_at(a, i);
             const int st = (int)(k % NS);
             const uint32_t ph = (uint32_t)(k / NS) & 1u;
             if (k >= NS) ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * st, ph ^ 1u));
@@ -732,7 +801,10 @@ __global__ void __launch_bounds__(FD_THREADS, 1) dd_dms_f32_ws(const FdArgs a)
 
     /* ---------------------------- summing warps ---------------------------- */
     long long k = 0;
-    for (long long item = blockIdx.x; item < a.nitems; item += grid, k++) {
+    long long ahead = blockIdx.x < nitems ? item_at(a, blockIdx.x) : 0;
+    for (long long i = blockIdx.x; i < nitems; i += grid, k++) {
+        const long long item = ahead;
+        if (i + grid < nitems) ahead = item_at(a, i + grid);
         const int st = (int)(k % NS);
         const uint32_t ph = (uint32_t)(k / NS) & 1u;
         if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * st, ph))) {
@@ -803,6 +875,61 @@ __global__ void __launch_bounds__(FD_THREADS, 1) dd_dms_f32_ws(const FdArgs a)
     }
 }
 
+/* ---------------------------------------------------------------- */
+/* Which items of a clipped run need FP32                            */
+/* ---------------------------------------------------------------- */
+/* A sum without a replaced spectrum in it is a sum of integers below 2^24: the
+ * FP32 result in any order, and what the integer stages give.  So a clipped run
+ * takes the FP32 stages only for the DM items whose windows reach a flagged
+ * spectrum, and the integer stages for the rest.  Interference is rare: 12
+ * bursts in 300 k spectra leave 8 % of the items, and the two stages took 1165 +
+ * 383 us in FP32 where they take MEASURED_CLIP now.  When every spectrum is flagged the
+ * integer stages have no items. */
+struct ClipPlan {
+    const uint8_t *flags;
+    long long nflags;
+    uint8_t *any;             /* [nblk] a flagged spectrum among 256 */
+    long long nblk;
+    long long ntile, nout;
+    int gmax, ng;             /* DMs a decision covers, and how many decisions a tile */
+    const int2 *range;        /* [ng] lowest and highest offset of those DMs */
+    int halo;
+    int gu, ngu, gf, ngf;     /* group sizes and counts of the integer and FP32 items */
+    int *list_u, *list_f, *cnt;       /* cnt: integer, FP32 items */
+    uint8_t *need_u, *need_f;         /* [nblk_s] subband tiles they read */
+    long long nblk_s;
+};
+
+__global__ void __launch_bounds__(256) dd_clip_any(const ClipPlan p)
+{
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int f = __syncthreads_or(i < p.nflags && p.flags[i]);
+    if (threadIdx.x == 0) p.any[blockIdx.x] = f ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(256) dd_clip_items(const ClipPlan p)
+{
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= p.ntile * p.ng) return;
+    const long long tile = i / p.ng;
+    const int g = (int)(i - tile * p.ng);
+    const int2 r = p.range[g];
+    const long long T0 = tile * DM_TILE;
+    /* spectra the tile's samples are made of: offset plus channel delay */
+    const long long b0 = (T0 + r.x) >> 8, b1 = min(p.nblk - 1, (T0 + DM_TILE - 1 + r.y + p.halo) >> 8);
+    bool hit = false;
+    for (long long b = b0; b <= b1 && !hit; b++) hit = p.any[b] != 0;
+    const long long s1 = min(p.nblk_s - 1, (T0 + DM_TILE - 1 + r.y) >> 8);
+    uint8_t *need = hit ? p.need_f : p.need_u;
+    for (long long b = b0; b <= s1; b++) need[b] = 1;
+    const int gs = hit ? p.gf : p.gu, ngs = hit ? p.ngf : p.ngu;
+    const int first = g * (p.gmax / gs), n = min(p.gmax / gs, ngs - first);
+    if (n <= 0) return;
+    const int at = atomicAdd(p.cnt + (hit ? 1 : 0), n);
+    int *list = hit ? p.list_f : p.list_u;
+    for (int k = 0; k < n; k++) list[at + k] = (int)(tile * ngs + first + k);
+}
+
 }  // namespace dd
 
 /* ---------------------------------------------------------------- */
@@ -825,6 +952,11 @@ struct CsDedisp {
     int *d_err = nullptr;          /* set by a DM-stage wait that gave up */
     uint32_t *d_sub = nullptr;
     float *d_subf = nullptr;       /* S of clipped runs (allocated by the first one) */
+    /* which of a clipped run's items need FP32 (allocated with d_subf) */
+    uint8_t *d_clip = nullptr;     /* counts, tile needs, flagged blocks, the two lists */
+    int2 *d_range = nullptr;       /* offsets of gmax DMs */
+    int gmax = 0, ngmax = 0;       /* 0: every item in FP32 */
+    std::vector<int2> range;
     int2 *d_fwin = nullptr;        /* clipped DM stage (rounds kernel): per (DM group, subband)
                                       window */
     int fwmax = 0;                 /* widest such window (floats) */
@@ -852,6 +984,8 @@ static void dd_release(CsDedisp *D)
     cudaFree(D->d_err);
     cudaFree(D->d_sub);
     cudaFree(D->d_subf);
+    cudaFree(D->d_clip);
+    cudaFree(D->d_range);
     cudaFree(D->d_fwin);
     cudaFree(D->d_fwin2);
     cudaFree(D->d_fcode);
@@ -1113,6 +1247,20 @@ CS_EXPORT CsDedisp *cs_dedisp_create(int nchan, int nsub, int ndm, const int *id
                     }
         }
     }
+    if (D->G > 0 && D->fG > 0) {
+        D->gmax = std::max(D->G, D->fG);            /* powers of two: one divides the other */
+        D->ngmax = (ndm + D->gmax - 1) / D->gmax;
+        D->range.resize(D->ngmax);
+        for (int g = 0; g < D->ngmax; g++) {
+            int lo = 1 << 30, hi = 0;
+            for (int d = g * D->gmax; d < std::min(ndm, (g + 1) * D->gmax); d++)
+                for (int q = 0; q < nsub; q++) {
+                    lo = std::min(lo, offsets[(size_t)d * nsub + q]);
+                    hi = std::max(hi, offsets[(size_t)d * nsub + q]);
+                }
+            D->range[g] = make_int2(lo, hi);
+        }
+    }
     if (sb_smem(D, 1) > max_optin) {
         fprintf(stderr, "Error: cs_dedisp_create: channel delays of %d samples need more "
                         "shared memory than a CTA has\n", halo);
@@ -1194,6 +1342,10 @@ CS_EXPORT CsDedisp *cs_dedisp_create(int nchan, int nsub, int ndm, const int *id
                                   4 * D->nstage * D->stage_words));
     DDCK(cudaFuncSetAttribute(dd::dd_subband_u8, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               max_optin));
+    DDCK(cudaFuncSetAttribute(dd::dd_subband_u8_256<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              max_optin));
+    DDCK(cudaFuncSetAttribute(dd::dd_subband_u8_256<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              max_optin));
     DDCK(cudaFuncSetAttribute(dd::dd_subband_clip, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               max_optin));
     /* a copy from pageable memory may return before its DMA lands; finish
@@ -1223,6 +1375,53 @@ static int dd_clip_rounds(const CsDedisp *D)
     return 0;
 }
 
+/* The room a clipped run's plan takes for the longest input: counts, needs of
+ * the subband tiles (integer, FP32), flagged blocks, then the item lists. */
+struct ClipRoom {
+    long long nblk, nblk_s, need_u, need_f, any, list_u, list_f, bytes;
+};
+
+static ClipRoom dd_clip_room(const CsDedisp *D)
+{
+    ClipRoom r;
+    const long long ntile = (D->max_spectra + dd::DM_TILE - 1) / dd::DM_TILE;
+    r.nblk = (D->max_spectra + 255) / 256 + 1;
+    r.nblk_s = D->sstride / 256 + 1;
+    r.need_u = 16;
+    r.need_f = r.need_u + r.nblk_s;
+    r.any = r.need_f + r.nblk_s;
+    r.list_u = (r.any + r.nblk + 15) / 16 * 16;
+    r.list_f = r.list_u + 4 * ntile * D->ngroups;
+    r.bytes = r.list_f + 4 * ntile * D->fngroups;
+    return r;
+}
+
+/* The subband stage of one kind over the tiles up to sfill. */
+static cudaError_t dd_subbands(CsDedisp *D, dd::SubArgs sa, bool clip, long long sfill,
+                               cudaStream_t st)
+{
+    int max_optin = 0;
+    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, D->device);
+    int slab = std::max(1, std::min(D->nsub, 256 / std::max(1, D->cps)));
+    while (slab > 1 && sb_smem(D, slab, clip) > std::min(max_optin, 100 * 1024)) slab /= 2;
+    sa.slab = slab;
+    sa.rowstride = sb_rowstride(D, slab);
+    sa.table_off = sb_table_offset(D, slab);
+    sa.flag_off = sb_flag_offset(D, slab);
+    const dim3 gs((D->nsub + slab - 1) / slab, (unsigned)((sfill + dd::SB_TT - 1) / dd::SB_TT));
+    const int smem = sb_smem(D, slab, clip);
+    const bool whole = slab * D->cps == 256 && D->nsub % slab == 0;
+    if (clip)
+        dd::dd_subband_clip<<<gs, dd::SB_THREADS, smem, st>>>(sa);
+    else if (whole && D->cps == 16)
+        dd::dd_subband_u8_256<16><<<gs, dd::SB_THREADS, smem, st>>>(sa);
+    else if (whole && D->cps == 8)
+        dd::dd_subband_u8_256<8><<<gs, dd::SB_THREADS, smem, st>>>(sa);
+    else
+        dd::dd_subband_u8<<<gs, dd::SB_THREADS, smem, st>>>(sa);
+    return cudaGetLastError();
+}
+
 static cudaError_t dd_enqueue(CsDedisp *D, const uint8_t *d_raw, long long nspec, long long nout,
                               float *d_out, long long ostride, cudaStream_t st,
                               const uint8_t *d_flags = nullptr, const float *d_levels = nullptr)
@@ -1232,20 +1431,14 @@ static cudaError_t dd_enqueue(CsDedisp *D, const uint8_t *d_raw, long long nspec
     /* subband stage over every sample the DM stage can read */
     const long long ntile_dm = (nout + dd::DM_TILE - 1) / dd::DM_TILE;
     const long long sfill = std::min(D->sstride, ntile_dm * dd::DM_TILE + D->maxoff + 64);
-    int max_optin = 0;
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, D->device);
-    int slab = std::max(1, std::min(D->nsub, 256 / std::max(1, D->cps)));
-    while (slab > 1 && sb_smem(D, slab, clip) > std::min(max_optin, 100 * 1024)) slab /= 2;
     dd::SubArgs sa;
+    memset(&sa, 0, sizeof(sa));
     sa.raw = d_raw;
     sa.nspec = nspec;
     sa.nchan = D->nchan;
     sa.cps = D->cps;
     sa.nsub = D->nsub;
-    sa.slab = slab;
     sa.halo = D->halo;
-    sa.rowstride = sb_rowstride(D, slab);
-    sa.table_off = sb_table_offset(D, slab);
     sa.idisp = D->d_idisp;
     sa.nvalid = nspec / D->L >= 1 ? (nspec / D->L - 1) * D->L : 0;
     sa.sfill = sfill;
@@ -1255,19 +1448,86 @@ static cudaError_t dd_enqueue(CsDedisp *D, const uint8_t *d_raw, long long nspec
     sa.nflags = nspec / D->L * D->L;
     sa.levels = d_levels;
     sa.L = D->L;
-    sa.flag_off = sb_flag_offset(D, slab);
     sa.subf = D->d_subf;
-    dim3 gs((D->nsub + slab - 1) / slab, (unsigned)((sfill + dd::SB_TT - 1) / dd::SB_TT));
+    const bool ws = clip && D->fG > 0 && !getenv("CS_B200_DEDISP_ROUNDS");
+    const bool split = ws && D->gmax > 0 && D->d_clip != nullptr;
     cudaError_t e = cudaMemsetAsync(D->d_err, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     cudaEventRecord(D->ev0, st);
-    if (clip)
-        dd::dd_subband_clip<<<gs, dd::SB_THREADS, sb_smem(D, slab, true), st>>>(sa);
-    else
-        dd::dd_subband_u8<<<gs, dd::SB_THREADS, sb_smem(D, slab), st>>>(sa);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (clip && D->fG > 0 && !getenv("CS_B200_DEDISP_ROUNDS")) {
+    const ClipRoom room = split ? dd_clip_room(D) : ClipRoom();
+    if (split) {
+        dd::ClipPlan p;
+        memset(&p, 0, sizeof(p));
+        if ((e = cudaMemsetAsync(D->d_clip, 0, room.list_u, st)) != cudaSuccess) return e;
+        p.flags = d_flags;
+        p.nflags = sa.nflags;
+        p.cnt = (int *)D->d_clip;
+        p.any = D->d_clip + room.any;
+        p.nblk = (sa.nflags + 255) / 256;
+        p.ntile = ntile_dm;
+        p.gmax = D->gmax;
+        p.ng = D->ngmax;
+        p.range = D->d_range;
+        p.halo = D->halo;
+        p.gu = D->G;
+        p.ngu = D->ngroups;
+        p.gf = D->fG;
+        p.ngf = D->fngroups;
+        p.list_u = (int *)(D->d_clip + room.list_u);
+        p.list_f = (int *)(D->d_clip + room.list_f);
+        p.need_u = D->d_clip + room.need_u;
+        p.need_f = D->d_clip + room.need_f;
+        p.nblk_s = room.nblk_s;
+        dd::dd_clip_any<<<(unsigned)p.nblk, 256, 0, st>>>(p);
+        dd::dd_clip_items<<<(unsigned)((ntile_dm * D->ngmax + 255) / 256), 256, 0, st>>>(p);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        sa.need = p.need_u;
+        if ((e = dd_subbands(D, sa, false, sfill, st)) != cudaSuccess) return e;
+        sa.need = p.need_f;
+    }
+    if ((e = dd_subbands(D, sa, clip, sfill, st)) != cudaSuccess) return e;
+    cudaEventRecord(D->ev1, st);
+    int nsm = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, D->device);
+    if (!clip || split) {
+        dd::DmArgs da;
+        memset(&da, 0, sizeof(da));
+        da.sub = D->d_sub;
+        da.sstride = D->sstride;
+        da.nsub = D->nsub;
+        da.nsub8 = D->nsub8;
+        da.ndm = D->ndm;
+        da.G = D->G;
+        da.ngroups = D->ngroups;
+        da.offs = D->d_offs;
+        da.flush = D->flush;
+        da.win = D->d_win;
+        da.code = D->d_code;
+        da.gbytes = D->d_gbytes;
+        da.code_bytes = D->code_bytes;
+        da.code_word = D->code_word;
+        da.zero_word = D->zero_word;
+        da.stage_words = D->stage_words;
+        da.nstage = D->nstage;
+        da.nitems = ntile_dm * D->ngroups;
+        if (split) {
+            da.count = (const int *)D->d_clip;
+            da.list = (const int *)(D->d_clip + room.list_u);
+        }
+        da.nout = nout;
+        da.out = d_out;
+        da.ostride = ostride;
+        da.err = D->d_err;
+        if (D->G > 0) {
+            const long long grid = std::min<long long>(da.nitems, nsm);
+            dd::dd_dms_u16<<<(unsigned)grid, dd::DM_THREADS, 4 * D->nstage * D->stage_words, st>>>(da);
+        } else {
+            dim3 gd((unsigned)((nout + 255) / 256), (unsigned)D->ndm);
+            dd::dd_dms_u16_direct<<<gd, 256, 0, st>>>(da);
+        }
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (ws) {
         dd::FdArgs fa;
         memset(&fa, 0, sizeof(fa));
         fa.sub = D->d_subf;
@@ -1285,62 +1545,23 @@ static cudaError_t dd_enqueue(CsDedisp *D, const uint8_t *d_raw, long long nspec
         fa.stage_words = D->fstage_words;
         fa.nstage = D->fnstage;
         fa.nitems = (nout + dd::FD_T - 1) / dd::FD_T * D->fngroups;
+        if (split) {
+            fa.count = (const int *)D->d_clip + 1;
+            fa.list = (const int *)(D->d_clip + room.list_f);
+        }
         fa.nout = nout;
         fa.out = d_out;
         fa.ostride = ostride;
         fa.err = D->d_err;
-        int nsm = 0;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, D->device);
         const long long grid = std::min<long long>(fa.nitems, nsm);
-        cudaEventRecord(D->ev1, st);
         dd::dd_dms_f32_ws<<<(unsigned)grid, dd::FD_THREADS, 4 * D->fnstage * D->fstage_words, st>>>(fa);
-        cudaEventRecord(D->ev2, st);
-        return cudaGetLastError();
-    }
-    if (clip) {
+    } else if (clip) {
         const long long ntile = (nout + dd::FT - 1) / dd::FT;
         const long long ngrp = (D->ndm + dd::FG - 1) / dd::FG;
         const int fr = dd_clip_rounds(D);
-        cudaEventRecord(D->ev1, st);
         dd::dd_dms_f32<<<(unsigned)(ntile * ngrp), 256, dd_clip_smem(fr, D->fwmax), st>>>(
             D->d_subf, D->sstride, D->nsub, D->ndm, D->d_offs, D->d_fwin, D->fwmax, fr, sfill,
             nout, d_out, ostride);
-        cudaEventRecord(D->ev2, st);
-        return cudaGetLastError();
-    }
-    dd::DmArgs da;
-    memset(&da, 0, sizeof(da));
-    da.sub = D->d_sub;
-    da.sstride = D->sstride;
-    da.nsub = D->nsub;
-    da.nsub8 = D->nsub8;
-    da.ndm = D->ndm;
-    da.G = D->G;
-    da.ngroups = D->ngroups;
-    da.offs = D->d_offs;
-    da.flush = D->flush;
-    da.win = D->d_win;
-    da.code = D->d_code;
-    da.gbytes = D->d_gbytes;
-    da.code_bytes = D->code_bytes;
-    da.code_word = D->code_word;
-    da.zero_word = D->zero_word;
-    da.stage_words = D->stage_words;
-    da.nstage = D->nstage;
-    da.nitems = ntile_dm * D->ngroups;
-    da.nout = nout;
-    da.out = d_out;
-    da.ostride = ostride;
-    da.err = D->d_err;
-    cudaEventRecord(D->ev1, st);
-    if (D->G > 0) {
-        int nsm = 0;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, D->device);
-        const long long grid = std::min<long long>(da.nitems, nsm);
-        dd::dd_dms_u16<<<(unsigned)grid, dd::DM_THREADS, 4 * D->nstage * D->stage_words, st>>>(da);
-    } else {
-        dim3 gd((unsigned)((nout + 255) / 256), (unsigned)D->ndm);
-        dd::dd_dms_u16_direct<<<gd, 256, 0, st>>>(da);
     }
     cudaEventRecord(D->ev2, st);
     return cudaGetLastError();
@@ -1432,6 +1653,23 @@ CS_EXPORT int cs_dedisp_run_device_clipped(CsDedisp *D, const uint8_t *d_raw, lo
         e = cudaMalloc((void **)&D->d_subf, sizeof(float) * (size_t)D->nsub * D->sstride);
         if (e == cudaSuccess)
             e = cudaMemset(D->d_subf, 0, sizeof(float) * (size_t)D->nsub * D->sstride);
+    }
+    /* the plan of which items need it; without room for it all of them do */
+    if (e == cudaSuccess && D->gmax > 0 && !D->d_clip) {
+        const long long items = (D->max_spectra + dd::DM_TILE - 1) / dd::DM_TILE *
+                                std::max(D->ngroups, D->fngroups);
+        if (items < 2147483647LL &&
+            cudaMalloc((void **)&D->d_clip, (size_t)dd_clip_room(D).bytes) == cudaSuccess &&
+            cudaMalloc((void **)&D->d_range, sizeof(int2) * D->range.size()) == cudaSuccess) {
+            e = cudaMemcpy(D->d_range, D->range.data(), sizeof(int2) * D->range.size(),
+                           cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = cudaDeviceSynchronize();  /* before a run on any stream */
+        } else {
+            (void)cudaGetLastError();
+            cudaFree(D->d_clip);
+            D->d_clip = nullptr;
+            D->gmax = 0;
+        }
     }
     cudaStream_t st = stream ? (cudaStream_t)stream : D->st;
     if (e == cudaSuccess) e = dd_enqueue(D, d_raw, nspec, nout, d_out, out_stride, st, d_flags,
