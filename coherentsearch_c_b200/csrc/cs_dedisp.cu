@@ -69,6 +69,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "cs_b200.h"
@@ -107,11 +108,26 @@ static __device__ __forceinline__ uint32_t smem_addr(const void *p)
 
 /* Asynchronous global -> shared copies (no register round trip, so all of
  * a thread's copies are in flight together); nbytes 0 writes zeros. */
+static __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, int nbytes)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(nbytes)
+                 : "memory");
+}
+
 static __device__ __forceinline__ void cp_async4(void *dst, const void *src, int nbytes)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src),
-                 "r"(nbytes)
-                 : "memory");
+    cp_async4(smem_addr(dst), src, nbytes);
+}
+
+/* The byte at a shared address plus a constant.  Not volatile, so that a sum's
+ * loads can be scheduled together: the addresses come from a table that is read
+ * after the barrier behind the staging. */
+template <int OFF>
+static __device__ __forceinline__ uint32_t lds_u8(uint32_t addr)
+{
+    uint32_t v;
+    asm("ld.shared.u8 %0, [%1 + %2];" : "=r"(v) : "r"(addr), "n"(OFF));
+    return v;
 }
 
 static __device__ __forceinline__ void cp_async16(void *dst, const void *src)
@@ -232,12 +248,20 @@ static __device__ __forceinline__ void sb_stage(const SubArgs &a, unsigned char 
         const int rpp = blockDim.x / wpr;                 /* rows per pass */
         const int w = threadIdx.x % wpr;
         if (threadIdx.x < rpp * wpr) {
-            const unsigned char *src = a.raw + T0 * a.nchan + col0 + 4 * w;
-            unsigned char *dst = sm + 4 * w;
-            for (int r = threadIdx.x / wpr; r < rows; r += rpp) {
-                const bool in = T0 + r < a.nspec;
-                cp_async4(dst + (size_t)r * a.rowstride, in ? src + (long long)r * a.nchan : a.raw,
-                          in ? 4 : 0);
+            const int r0 = threadIdx.x / wpr;
+            const unsigned char *src = a.raw + (T0 + r0) * a.nchan + col0 + 4 * w;
+            const long long sstep = (long long)rpp * a.nchan;
+            uint32_t dst = smem_addr(sm) + 4 * w + r0 * a.rowstride;
+            const uint32_t dstep = (uint32_t)(rpp * a.rowstride);
+            if (T0 + rows <= a.nspec) {
+#pragma unroll 4
+                for (int r = r0; r < rows; r += rpp, src += sstep, dst += dstep)
+                    cp_async4(dst, src, 4);
+            } else {
+                for (int r = r0; r < rows; r += rpp, src += sstep, dst += dstep) {
+                    const bool in = T0 + r < a.nspec;
+                    cp_async4(dst, in ? src : a.raw, in ? 4 : 0);
+                }
             }
         }
         cp_async_wait_all();
@@ -291,8 +315,26 @@ __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8(const SubArgs a)
  * shared load and half an addition (the general kernel also reads the offset and
  * adds it), and writes both halves of a word at once where it has them.  Bound by
  * the shared loads and the staging; 500 k spectra of 1024 channels: 253 us in
- * the general kernel, MEASURED_SB here, 79 us for the bytes read. */
+ * the general kernel, 187 here, 79 us for the bytes read. */
 constexpr int SB_RS = 260;
+
+template <int CPS, int G>
+static __device__ __forceinline__ uint32_t sum_group(const uint32_t (&base)[CPS])
+{
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < CPS; k += 2)
+        s += lds_u8<G * 32 * SB_RS>(base[k]) + lds_u8<G * 32 * SB_RS>(base[k + 1]);
+    return s;
+}
+
+template <int CPS, int NG, int... G>
+static __device__ __forceinline__ void sum_groups(const uint32_t (&base)[CPS], uint32_t (&acc)[NG],
+                                                  std::integer_sequence<int, G...>)
+{
+    ((acc[G] = sum_group<CPS, G>(base)), ...);
+}
+
 template <int CPS>
 __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8_256(const SubArgs a)
 {
@@ -306,18 +348,15 @@ __global__ void __launch_bounds__(SB_THREADS) dd_subband_u8_256(const SubArgs a)
     constexpr int NG = SB_TT / 32, HG = DM_P / 32;
     static_assert(NG == 2 * HG, "a tile is both halves of its first words");
     for (int sl = warp; sl < a.slab; sl += SB_THREADS / 32) {
-        const unsigned char *base[CPS];
+        uint32_t base[CPS];
 #pragma unroll
-        for (int k = 0; k < CPS; k++) base[k] = sm + lane * SB_RS + coff[sl * CPS + k];
-        uint32_t acc[NG];
+        for (int k = 0; k < CPS; k++)
+            base[k] = smem_addr(sm) + (uint32_t)(lane * SB_RS + coff[sl * CPS + k]);
+        uint32_t acc[NG] = {};
+        sum_groups<CPS, NG>(base, acc, std::make_integer_sequence<int, NG>());
 #pragma unroll
-        for (int g = 0; g < NG; g++) {
-            acc[g] = 0;
-#pragma unroll
-            for (int k = 0; k < CPS; k += 2)
-                acc[g] += (uint32_t)base[k][g * 32 * SB_RS] + (uint32_t)base[k + 1][g * 32 * SB_RS];
+        for (int g = 0; g < NG; g++)
             if (T0 + g * 32 + lane >= a.nvalid) acc[g] = 0;
-        }
         uint32_t *row = a.sub + (long long)(s0 + sl) * a.sstride;
         uint16_t *row16 = reinterpret_cast<uint16_t *>(row);
 #pragma unroll
@@ -883,7 +922,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) dd_dms_f32_ws(const FdArgs a)
  * takes the FP32 stages only for the DM items whose windows reach a flagged
  * spectrum, and the integer stages for the rest.  Interference is rare: 12
  * bursts in 300 k spectra leave 8 % of the items, and the two stages took 1165 +
- * 383 us in FP32 where they take MEASURED_CLIP now.  When every spectrum is flagged the
+ * 383 us in FP32 where they take 612 + 121 us and 90 + 104 us now.  When every spectrum is flagged the
  * integer stages have no items. */
 struct ClipPlan {
     const uint8_t *flags;

@@ -5,7 +5,8 @@
  *   realfft   forward real FFT of the N samples, packed PRESTO-style:
  *             N/2 complex bins, bin 0 holding (DC, Nyquist)
  *             (src/datpipe.c:101-138).  The transform is cuFFT's R2C (a plain
- *             library FFT); the packing is a kernel here.
+ *             library FFT); its bins are the packed ones except bin 0, which
+ *             the normalisation replaces, so nothing is packed here.
  *   rednoise  the spectrum is normalised by running block medians of the
  *             power (src/datpipe.c:143-253): blocks of startwidth*ln(binnum)
  *             bins below endfreq Hz and endwidth bins above; a block's noise
@@ -57,14 +58,6 @@ static __device__ __forceinline__ float presto_invsqrtf(float x)
     const float y = __int_as_float(0x5f3759df - (__float_as_int(x) >> 1));
     const float t = __fmul_rn(__fmul_rn(0.5f, x), y);
     return __fmul_rn(y, __fmaf_rn(-t, y, 1.5f));
-}
-
-/* R2C output (N/2 + 1 bins) -> PRESTO packing (N/2 bins, bin 0 = DC, Nyq). */
-__global__ void pack_kernel(const float2 *X, float2 *out, long long n2)
-{
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n2) return;
-    out[k] = k == 0 ? make_float2(X[0].x, X[n2].x) : X[k];
 }
 
 /* One warp per block: level = (float)(lower median power / ln 2).  The
@@ -137,45 +130,58 @@ __global__ void slope_kernel(const float *level, const int *blen, int nblk, floa
                        (0.5 * (double)(blen[b - 1] + blen[b])));
 }
 
-/* One thread per bin.  Segment s: first bin sstart[s], level index
- * slvl[s]; sslope[s] = -1 for the first half block (no slope), 0 for a
- * slope of 1.0, else the block whose slope applies. */
-__global__ void normalise_kernel(const float2 *amps, float2 *out, long long n2,
-                                 const long long *sstart, const int *slvl, const int *sslope,
-                                 int nseg, const float *level, const float *slope)
+/* Two bins a thread.  Segment s: first bin sstart[s], level index slvl[s];
+ * sslope[s] = -1 for the first half block (no slope), 0 for a slope of 1.0, else
+ * the block whose slope applies.  From segment `us` on the blocks all have
+ * `width` bins (rednoise's endwidth, above endfreq; the last block may be
+ * shorter), so a bin's segment is a division; the few thousand bins before are
+ * searched.  amps is the R2C output as it is: only bin 0 differs in the packed
+ * spectrum, and it becomes (1, 0).  Bound by the bytes (33 MB at 4.1 M points: 5
+ * us); one thread a CTA searching all segments for its 256 bins, with a packing
+ * pass before, took 27 + 6.5 us, this 10. */
+__global__ void __launch_bounds__(256) normalise_kernel(const float2 *amps, float2 *out,
+                                                        long long n2, const long long *sstart,
+                                                        const int *slvl, const int *sslope,
+                                                        int nseg, int us, int width,
+                                                        const float *level, const float *slope)
 {
-    /* the segment of the CTA's first bin, found once; a CTA's bins span a
-     * few segments, so each thread walks on from there */
-    __shared__ int seg0;
-    const long long k0 = (long long)blockIdx.x * blockDim.x;
-    if (threadIdx.x == 0) {
-        int lo = 0, hi = nseg - 1;
-        while (lo < hi) {             /* last segment starting at or before k0 */
-            const int mid = (lo + hi + 1) >> 1;
-            if (sstart[mid] <= k0) lo = mid;
-            else hi = mid - 1;
+    const long long b0 = (long long)blockIdx.x * 512 + threadIdx.x;
+    const long long ustart = __ldg(sstart + us);
+    float2 v[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        v[u] = b0 + 256 * u < n2 ? amps[b0 + 256 * u] : make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const long long k = b0 + 256 * u;
+        if (k >= n2) break;
+        if (k == 0) {
+            out[0] = make_float2(1.0f, 0.0f);
+            continue;
         }
-        seg0 = lo;
+        int lo = 0;
+        if (k >= ustart) {
+            lo = us + (int)((k - ustart) / width);
+            if (lo >= nseg - 2) lo = nseg - 2 + (k >= __ldg(sstart + nseg - 1) ? 1 : 0);
+        } else {
+            int hi = us;
+            while (lo < hi) {                   /* last segment starting at or before k */
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(sstart + mid) <= k) lo = mid;
+                else hi = mid - 1;
+            }
+        }
+        const float lv = __ldg(level + __ldg(slvl + lo));
+        const int si = __ldg(sslope + lo);
+        float norm;
+        if (si < 0) {
+            norm = presto_invsqrtf(lv);
+        } else {
+            const float sl = si == 0 ? 1.0f : __ldg(slope + si);
+            norm = presto_invsqrtf(__fmaf_rn(sl, (float)(k - __ldg(sstart + lo)), lv));
+        }
+        out[k] = make_float2(__fmul_rn(v[u].x, norm), __fmul_rn(v[u].y, norm));
     }
-    __syncthreads();
-    const long long k = k0 + threadIdx.x;
-    if (k >= n2) return;
-    if (k == 0) {
-        out[0] = make_float2(1.0f, 0.0f);
-        return;
-    }
-    int lo = seg0;
-    while (lo + 1 < nseg && sstart[lo + 1] <= k) lo++;
-    const float lv = level[slvl[lo]];
-    float norm;
-    if (sslope[lo] < 0) {
-        norm = presto_invsqrtf(lv);
-    } else {
-        const float sl = sslope[lo] == 0 ? 1.0f : slope[sslope[lo]];
-        norm = presto_invsqrtf(__fmaf_rn(sl, (float)(k - sstart[lo]), lv));
-    }
-    const float2 v = amps[k];
-    out[k] = make_float2(__fmul_rn(v.x, norm), __fmul_rn(v.y, norm));
 }
 
 }  // namespace sp
@@ -188,12 +194,12 @@ struct CsSpectrum {
     bool planned = false;
     float *d_series = nullptr;     /* staging for the host entry point */
     float2 *d_X = nullptr;         /* R2C output, N/2 + 1 bins */
-    float2 *d_pack = nullptr;      /* packed, before normalisation */
     float2 *d_out = nullptr;       /* staging for the host entry point */
     long long *d_bstart = nullptr, *d_sstart = nullptr;
     int *d_blen = nullptr, *d_slvl = nullptr, *d_sslope = nullptr;
     float *d_level = nullptr, *d_slope = nullptr;
     int nblk = 0, nseg = 0;
+    int useg = 0, uwidth = 1;      /* segments from useg on are uwidth bins apart */
     cudaStream_t st = nullptr;
 };
 
@@ -203,7 +209,6 @@ static void spec_release(CsSpectrum *S)
     if (S->planned) cufftDestroy(S->plan);
     cudaFree(S->d_series);
     cudaFree(S->d_X);
-    cudaFree(S->d_pack);
     cudaFree(S->d_out);
     cudaFree(S->d_bstart);
     cudaFree(S->d_sstart);
@@ -299,6 +304,11 @@ CS_EXPORT CsSpectrum *cs_spectrum_create(long long N, double dt, int startwidth,
     S->dt = dt;
     S->nblk = nblk;
     S->nseg = (int)sstart.size();
+    /* the run of endwidth steps up to the last segment but one (the last step is
+     * at most that); nseg >= 2 */
+    S->uwidth = endwidth;
+    S->useg = S->nseg - 2;
+    while (S->useg > 0 && sstart[S->useg] - sstart[S->useg - 1] == endwidth) S->useg--;
 #define SPCK(x)                                                                        \
     do {                                                                               \
         cudaError_t e_ = (x);                                                          \
@@ -311,7 +321,6 @@ CS_EXPORT CsSpectrum *cs_spectrum_create(long long N, double dt, int startwidth,
     SPCK(cudaSetDevice(device));
     SPCK(cudaStreamCreateWithFlags(&S->st, cudaStreamNonBlocking));
     SPCK(cudaMalloc((void **)&S->d_X, sizeof(float2) * (size_t)(n2 + 1)));
-    SPCK(cudaMalloc((void **)&S->d_pack, sizeof(float2) * (size_t)n2));
     SPCK(cudaMalloc((void **)&S->d_bstart, sizeof(long long) * nblk));
     SPCK(cudaMalloc((void **)&S->d_blen, sizeof(int) * nblk));
     SPCK(cudaMalloc((void **)&S->d_level, sizeof(float) * nblk));
@@ -347,14 +356,13 @@ static cudaError_t spec_enqueue(CsSpectrum *S, const float *d_series, float2 *d_
         cufftExecR2C(S->plan, (cufftReal *)d_series, (cufftComplex *)S->d_X) != CUFFT_SUCCESS)
         return cudaErrorLaunchFailure;
     const long long n2 = S->n2;
-    const unsigned g = (unsigned)((n2 + 255) / 256);
-    sp::pack_kernel<<<g, 256, 0, st>>>(S->d_X, S->d_pack, n2);
-    sp::block_level_kernel<<<(S->nblk + 7) / 8, 256, 0, st>>>(S->d_pack, S->d_bstart, S->d_blen,
+    sp::block_level_kernel<<<(S->nblk + 7) / 8, 256, 0, st>>>(S->d_X, S->d_bstart, S->d_blen,
                                                                S->nblk, log(2.0), S->d_level);
     sp::slope_kernel<<<(S->nblk + 255) / 256, 256, 0, st>>>(S->d_level, S->d_blen, S->nblk,
                                                            S->d_slope);
-    sp::normalise_kernel<<<g, 256, 0, st>>>(S->d_pack, d_amps, n2, S->d_sstart, S->d_slvl,
-                                            S->d_sslope, S->nseg, S->d_level, S->d_slope);
+    sp::normalise_kernel<<<(unsigned)((n2 + 511) / 512), 256, 0, st>>>(
+        S->d_X, d_amps, n2, S->d_sstart, S->d_slvl, S->d_sslope, S->nseg, S->useg, S->uwidth,
+        S->d_level, S->d_slope);
     return cudaGetLastError();
 }
 
