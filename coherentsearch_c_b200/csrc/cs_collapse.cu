@@ -25,6 +25,9 @@
  *                    sort gives (kept candidates never tie in frequency:
  *                    equal frequencies are related with m = n = 1).
  *
+ * remove without a sort at all: bins along r (bin_kernel).  What follows is
+ * the way without remove and where the bins would be too many.
+ *
  * Ordering without a sort on r: within one decimation slot, r (and freq)
  * rises strictly with the trial index, so a CUB radix sort on (slot, chunk,
  * j) lines every slot up in r order, and a merge places each candidate at
@@ -327,6 +330,148 @@ static __device__ __forceinline__ Candidate make_cand(double r, double freq, dou
     return c;
 }
 
+/* ---- remove_duplicates without a sort ----
+ * Bins of just under dr_tol along r: two records of one bin always belong to
+ * one run, two with two empty bins between them never do, and neighbours are
+ * decided by the largest r of the one and the smallest of the other, which are
+ * the two values the sorted list would compare.  So a run is a stretch of bins,
+ * and its first member of largest metric is the first of its bins' bests.  Four
+ * kernels and one memset on the list take the place of the radix sort on
+ * (slot, chunk, j), the merge of the slots and the scan: launches are what a list
+ * of some ten thousand records costs.  (A list of 10 k records from 150 k points:
+ * 100 -> 33 us of kernels; 32 of them with their searches 6.4 -> 4.5 ms.) */
+constexpr int BT = 1024;                /* bins in a block */
+constexpr unsigned NONE = 0xFFFFFFFFu;
+constexpr unsigned long long BINS_PER_REC = 1024, BINS_MOST = 1u << 24;
+
+struct Bins {                           /* all ones before a list */
+    unsigned long long *best;           /* [n] by run: inverted (metric, earliest bin) */
+    unsigned long long *lo, *nhi;       /* [nb] bits of the smallest r; inverted, of the largest */
+    unsigned *idx;                      /* [nb] the first record of largest metric */
+    unsigned *starts;                   /* bit per bin: a run starts there */
+    unsigned *cnt;                      /* per block of BT bins: run starts */
+    unsigned nb;
+    double inv;                         /* bins per unit of r */
+};
+
+struct RecGeo {                         /* what gives a record its r */
+    const CsRec *recs;
+    const CsChunk *chunks;
+    SlotInfo si;
+    int nslot, nprof;
+    double r_lo, lodr, nyq, T, thr;
+};
+
+static __device__ __forceinline__ double rec_r(const RecGeo &g, const CsRec &rc)
+{
+    const double rstart = g.r_lo + (double)g.chunks[rc.chunk].i0 * g.lodr;
+    const double rfreq = rstart + (double)rc.j * g.lodr;
+    const double kmul = (double)g.si.k[rc.slot];
+    return kmul != 1.0 ? kmul * rfreq : rfreq;
+}
+
+/* Records to their bins.  The lists are short and in the L2: the chains of
+ * dependent reads bound it, so no value is written that is already beaten. */
+__global__ void __launch_bounds__(NT) bin_kernel(const __grid_constant__ RecGeo g, unsigned n,
+                                                 const __grid_constant__ Bins bn, double *r,
+                                                 double *freq, double *metric, int *nharm)
+{
+    const unsigned i = blockIdx.x * NT + threadIdx.x;
+    if (i >= n) return;
+    const CsRec rc = g.recs[i];
+    if (!((double)rc.metric > g.thr) || rc.slot < 0 || rc.slot >= g.nslot) return;
+    const double x = rec_r(g, rc);
+    if (rc.slot != 0 && !(x < g.nyq)) return;
+    r[i] = x;
+    freq[i] = x / g.T;
+    metric[i] = (double)rc.metric;
+    nharm[i] = g.si.Hk[rc.slot];
+    const unsigned b = min((unsigned)(x * bn.inv), bn.nb - 1u);
+    const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
+    volatile const unsigned long long *lo = bn.lo, *nhi = bn.nhi;
+    if (xb < lo[b]) atomicMin(&bn.lo[b], xb);
+    if (~xb < nhi[b]) atomicMin(&bn.nhi[b], ~xb);
+    unsigned old = *(volatile unsigned *)&bn.idx[b];
+    for (;;) {
+        if (old != NONE) {
+            const CsRec ro = g.recs[old];
+            if (ro.metric > rc.metric) break;
+            if (ro.metric == rc.metric) {       /* the earlier in (r, chunk, slot, j) order */
+                const double xo = rec_r(g, ro);
+                if (xo < x) break;
+                if (xo == x && (ro.chunk < rc.chunk ||
+                                (ro.chunk == rc.chunk &&
+                                 (ro.slot < rc.slot || (ro.slot == rc.slot && ro.j <= rc.j)))))
+                    break;
+            }
+        }
+        const unsigned was = atomicCAS(&bn.idx[b], old, i);
+        if (was == old) break;
+        old = was;
+    }
+}
+
+/* The bins where a run starts: a word for every 32, their number for every BT. */
+__global__ void __launch_bounds__(BT) bin_starts_kernel(const __grid_constant__ Bins bn, double drtol)
+{
+    const unsigned b = blockIdx.x * BT + threadIdx.x;
+    bool start = false;
+    if (b < bn.nb && bn.idx[b] != NONE) {
+        start = true;
+        unsigned p = NONE;
+        if (b >= 1 && bn.idx[b - 1] != NONE) p = b - 1;
+        else if (b >= 2 && bn.idx[b - 2] != NONE) p = b - 2;
+        if (p != NONE)
+            start = __longlong_as_double((long long)bn.lo[b]) -
+                        __longlong_as_double((long long)~bn.nhi[p]) > drtol;
+    }
+    const unsigned w = __ballot_sync(0xffffffffu, start);
+    if ((threadIdx.x & 31) == 0) bn.starts[b >> 5] = w;
+    const int c = __syncthreads_count(start);
+    if (threadIdx.x == 0) bn.cnt[blockIdx.x] = (unsigned)c;
+}
+
+/* Every bin's best to its run; the number of runs to *m. */
+__global__ void __launch_bounds__(BT) bin_offer_kernel(const __grid_constant__ Bins bn,
+                                                       const CsRec *recs, unsigned *m)
+{
+    __shared__ unsigned wsum[BT / 32], wpre[BT / 32];
+    __shared__ unsigned base;
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned b = blockIdx.x * BT + threadIdx.x;
+    const unsigned word = bn.starts[b >> 5];
+    unsigned s = 0;                             /* the runs of the blocks before */
+    for (unsigned q = threadIdx.x; q < blockIdx.x; q += BT) s += bn.cnt[q];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) {
+        wsum[w] = s;
+        wpre[w] = __popc(word);
+    }
+    __syncthreads();
+    if (w == 0) {
+        const unsigned all = __reduce_add_sync(0xffffffffu, wsum[lane]);
+        const unsigned own = wpre[lane];
+        unsigned inc = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= (unsigned)d) inc += o;
+        }
+        wpre[lane] = inc - own;
+        if (lane == 0) base = all;
+        if (lane == 31 && blockIdx.x == gridDim.x - 1) *m = all + inc;
+    }
+    __syncthreads();
+    if (b >= bn.nb) return;
+    const unsigned x = bn.idx[b];
+    if (x == NONE) return;
+    const unsigned run = base + wpre[w] + __popc(word & (0xffffffffu >> (31 - lane))) - 1u;
+    const unsigned long long inv =
+        ~(((unsigned long long)ordered_bits(recs[x].metric + 0.0f) << 32) |
+          (unsigned long long)(0xFFFFFFFFu - b));
+    if (inv < *(volatile unsigned long long *)&bn.best[run]) atomicMin(&bn.best[run], inv);
+}
+
 struct FinishSmem {
     FinishShared f;
     union {
@@ -335,21 +480,27 @@ struct FinishSmem {
     } t;
 };
 
-/* The last steps for a list in global memory.  Lists past CAP are ranked by
- * counting and walked in global memory (the walk, not the ranking, is what they
- * cost). */
-__global__ void __launch_bounds__(FT) finish_kernel(const unsigned *list, const unsigned *mp,
+/* The last steps for a list in global memory, which the runs' bests give first
+ * when there are any.  Lists past CAP are ranked by counting and walked in global
+ * memory (the walk, not the ranking, is what they cost).  The first CAP of the
+ * result also go to pinned memory, with the number: no copy, and one wait less. */
+__global__ void __launch_bounds__(FT) finish_kernel(unsigned *list, const unsigned long long *best,
+                                                    const unsigned *bidx, const unsigned *mp,
                                                     int harm_remove, int numharm, double tol,
                                                     const double *r, const double *freq,
                                                     const double *metric, const int *nharm,
                                                     unsigned *mpos, unsigned char *removed,
                                                     unsigned char *keep, Candidate *out,
-                                                    unsigned *nout)
+                                                    Candidate *pinned, unsigned *nout)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
     FinishSmem &sm = *reinterpret_cast<FinishSmem *>(fsm);
     const unsigned m = *mp;
     const bool small = m <= CAP;
+    if (best) {
+        for (unsigned p = threadIdx.x; p < m; p += FT) list[p] = bidx[(unsigned)best[p]];
+        __syncthreads();
+    }
     if (harm_remove && small) {
         harmonics_keep(sm.f, sm.t.sort, m, numharm, tol, [&](unsigned p, float &mt, double &rr) {
             const unsigned c = list[p];
@@ -382,7 +533,9 @@ __global__ void __launch_bounds__(FT) finish_kernel(const unsigned *list, const 
         sm.f, m, [&](unsigned i) { return !harm_remove || (small ? sm.f.keep[i] : keep[i]); },
         [&](unsigned i, unsigned o) {
             const unsigned c = list[i];
-            out[o] = make_cand(r[c], freq[c], metric[c], nharm[c]);
+            const Candidate x = make_cand(r[c], freq[c], metric[c], nharm[c]);
+            out[o] = x;
+            if (o < CAP) pinned[o] = x;
         });
     if (threadIdx.x == 0) *nout = n;
 }
@@ -616,9 +769,11 @@ struct CsCollapse {
     unsigned *mpos;
     unsigned char *removed, *keep;
     Candidate *out;
-    unsigned *counters;             /* device: nvalid, runs, kept; then per-slot counts
-                                       and starts (CS_MAX_SLOT each) */
-    unsigned *h_counters;           /* pinned */
+    unsigned *counters;             /* device: valid, runs; then per-slot counts and
+                                       starts (CS_MAX_SLOT each) */
+    unsigned *h_counters;           /* pinned: the length of the list */
+    void *bins;                     /* Bins, for the longest list so far */
+    size_t bins_bytes;
     Candidate *h_out;               /* pinned */
     size_t h_out_cap;
     void *temp;
@@ -698,7 +853,7 @@ CsCollapse *cs_collapse_new(void)
 {
     CsCollapse *w = (CsCollapse *)calloc(1, sizeof(CsCollapse));
     if (!w) return nullptr;
-    /* one pinned block: the short path's list, then its status and the counters */
+    /* one pinned block: a short result, then its status and the length */
     if (cudaMallocHost((void **)&w->s_out, cl::CAP * sizeof(Candidate) + 8 * sizeof(unsigned)) !=
         cudaSuccess) {
         free(w);
@@ -714,6 +869,7 @@ void cs_collapse_free(CsCollapse *w)
     if (!w) return;
     collapse_release_buffers(w);
     cudaFree(w->counters);
+    cudaFree(w->bins);
     if (w->h_out) cudaFreeHost(w->h_out);
     if (w->s_out) cudaFreeHost(w->s_out);
     free(w);
@@ -784,6 +940,53 @@ int cs_collapse_small_status(const CsCollapse *w, unsigned *n, int *err)
     return w->s_status[3] ? 1 : 0;
 }
 
+/* The bins of a list, all ones, on the stream; false when the sort is the way.
+ * A bin is 20 bytes to clear and to read, a record about 100 in the sort's passes
+ * and its list some 20 launches.  Sort against bins, with both waits: 5 k records
+ * in 0.1, 0.5 and 4.2 M bins 156:78, 166:96 and 194:147 us, 80 k records in the
+ * same 267:105, 345:222 and 662:564.  The ends would meet near 2 k bins a record;
+ * BINS_MOST bounds the memory (336 MB).
+ * They are a millionth narrower than dr_tol; rounding of r and of its product
+ * with inv stays below that for up to 2^27 of them.  r >= 0 keeps the
+ * order of the bits. */
+static bool bins_for(CsCollapse *w, unsigned n, long long nchunks, const cl::SlotInfo &si,
+                     int nprof, double r_lo, double lodr, double N, double dr_tol, cudaStream_t st,
+                     cl::Bins &bn)
+{
+    if (!(dr_tol > 0.0) || !(r_lo >= 0.0) || !(lodr > 0.0)) return false;
+    const double width = dr_tol * (1.0 - 1e-6);
+    const double top = std::max(
+        N / 2.0, (r_lo + (double)nchunks * (double)nprof * lodr) * (double)si.k[0]);
+    const double want = top / width + 2.0;
+    const unsigned long long most =
+        std::min((unsigned long long)n * cl::BINS_PER_REC, cl::BINS_MOST);
+    if (!(want < (double)most)) return false;
+    bn.nb = (unsigned)want;
+    bn.inv = 1.0 / width;
+    const size_t pad = ((size_t)bn.nb + cl::BT - 1) / cl::BT * cl::BT, blocks = pad / cl::BT;
+    const size_t ones = ((size_t)n + 2 * (size_t)bn.nb) * sizeof(uint64_t) + (size_t)bn.nb * 4;
+    const size_t bytes = ones + pad / 8 + blocks * 4;
+    if (bytes > w->bins_bytes) {
+        cudaFree(w->bins);
+        w->bins = nullptr;
+        w->bins_bytes = 0;
+        const size_t c = bytes + (size_t)n * 2;     /* room for a quarter more records */
+        if (cudaMalloc(&w->bins, c) != cudaSuccess) {
+            cudaGetLastError();
+            w->bins = nullptr;
+            return false;
+        }
+        w->bins_bytes = c;
+    }
+    bn.best = (unsigned long long *)w->bins;
+    bn.lo = bn.best + n;
+    bn.nhi = bn.lo + bn.nb;
+    bn.idx = (unsigned *)(bn.nhi + bn.nb);
+    bn.starts = bn.idx + bn.nb;
+    bn.cnt = bn.starts + pad / 32;
+    return cudaMemsetAsync(w->bins, 0xFF, ones, st) == cudaSuccess;
+}
+
 int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsChunk *chunks,
                         long long nchunks, const int *slot_k, const int *slot_Hk, int nslot,
                         int nprof, double r_lo, double lodr, double N, double T,
@@ -798,77 +1001,84 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
     memset(&si, 0, sizeof(si));
     for (int s = 0; s < nslot; s++) { si.k[s] = slot_k[s]; si.Hk[s] = slot_Hk[s]; }
     const unsigned g = (n + cl::NT - 1) / cl::NT;
-    const int end_bit = bit_length_u64((uint64_t)nchunks * (uint64_t)nslot * (uint64_t)nprof);
-    size_t tb = 0;
-    const unsigned *order = nullptr, *listp = nullptr;
     cudaError_t e = collapse_reserve(w, n);       /* allocates the counters on first use */
-    if (e != cudaSuccess || !w->counters) {
+    if (e == cudaSuccess && !w->counters) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = finish_prepare();
+    if (e != cudaSuccess) {
         fprintf(stderr, "Error: candidate collapse on the GPU: %s\n", cudaGetErrorString(e));
         return -1;
     }
-    unsigned *nv = w->counters, *m = w->counters + 1, *nout = w->counters + 2;
-    e = cudaMemsetAsync(w->counters, 0, (4 + 2 * CS_MAX_SLOT) * sizeof(unsigned), st);
-    unsigned *slot_cnt = w->counters + 4, *slot_start = w->counters + 4 + CS_MAX_SLOT;
-    if (e == cudaSuccess) {
-        cl::harvest_kernel<<<g, cl::NT, 0, st>>>(recs, n, chunks, nchunks, si, nslot, nprof,
-                                                 r_lo, lodr, N / 2.0, T, threshold, w->key[0],
-                                                 w->bkey, w->slot_of, w->idx[0], w->r, w->freq,
-                                                 w->metric, w->nharm, nv, slot_cnt);
+    unsigned *nv = w->counters, *m = w->counters + 1;
+    cl::Bins bn;
+    unsigned *list = w->list;
+    const bool binned = remove && bins_for(w, n, nchunks, si, nprof, r_lo, lodr, N, dr_tol, st, bn);
+    if (binned) {
+        const cl::RecGeo geo = {recs, chunks, si, nslot, nprof, r_lo, lodr, N / 2.0, T, threshold};
+        const unsigned gb = (bn.nb + cl::BT - 1) / cl::BT;
+        cl::bin_kernel<<<g, cl::NT, 0, st>>>(geo, n, bn, w->r, w->freq, w->metric, w->nharm);
+        cl::bin_starts_kernel<<<gb, cl::BT, 0, st>>>(bn, dr_tol);
+        cl::bin_offer_kernel<<<gb, cl::BT, 0, st>>>(bn, recs, m);
         e = cudaGetLastError();
-    }
-    /* every slot's records in trial order; invalid records (all-ones key) last */
-    cub::DoubleBuffer<uint64_t> kb(w->key[0], w->key[1]);
-    cub::DoubleBuffer<unsigned> ib(w->idx[0], w->idx[1]);
-    if (e == cudaSuccess) {
-        tb = w->temp_bytes;
-        e = cub::DeviceRadixSort::SortPairs(w->temp, tb, kb, ib, (int)n, 0, end_bit, st);
-    }
-    /* merged into stable r order (remove) or stable frequency order */
-    if (e == cudaSuccess) {
-        cl::slot_starts_kernel<<<1, 1, 0, st>>>(slot_cnt, nslot, slot_start);
-        cl::merge_kernel<<<g, cl::NT, 0, st>>>(ib.Current(), nv, w->slot_of, w->bkey,
-                                               remove ? w->r : w->freq, slot_start, slot_cnt,
-                                               nslot, w->merged);
-        e = cudaGetLastError();
-    }
-    order = w->merged;
-    if (remove) {
-        if (e == cudaSuccess) {
-            cl::run_flags_kernel<<<g, cl::NT, 0, st>>>(order, w->r, n, nv, dr_tol, w->flag);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) {
-            tb = w->temp_bytes;
-            e = cub::DeviceScan::ExclusiveSum(w->temp, tb, w->flag, w->runid, (int)n, st);
-        }
-        /* the key buffers are free once the merge has run: best-of-run slots */
-        unsigned long long *best = reinterpret_cast<unsigned long long *>(w->key[0]);
-        if (e == cudaSuccess) e = cudaMemsetAsync(best, 0, (size_t)n * sizeof(uint64_t), st);
-        if (e == cudaSuccess) {
-            cl::count_runs_kernel<<<1, 1, 0, st>>>(w->flag, w->runid, n, m);
-            cl::run_offer_kernel<<<g, cl::NT, 0, st>>>(order, w->metric, w->flag, w->runid, nv,
-                                                       best);
-            cl::run_take_kernel<<<g, cl::NT, 0, st>>>(order, best, n, m, w->list);
-            e = cudaGetLastError();
-        }
-        listp = w->list;
     } else {
+        const int end_bit =
+            bit_length_u64((uint64_t)nchunks * (uint64_t)nslot * (uint64_t)nprof);
+        e = cudaMemsetAsync(w->counters, 0, (4 + 2 * CS_MAX_SLOT) * sizeof(unsigned), st);
+        unsigned *slot_cnt = w->counters + 4, *slot_start = w->counters + 4 + CS_MAX_SLOT;
         if (e == cudaSuccess) {
-            cl::copy_count_kernel<<<1, 1, 0, st>>>(nv, m);
+            cl::harvest_kernel<<<g, cl::NT, 0, st>>>(recs, n, chunks, nchunks, si, nslot, nprof,
+                                                     r_lo, lodr, N / 2.0, T, threshold, w->key[0],
+                                                     w->bkey, w->slot_of, w->idx[0], w->r, w->freq,
+                                                     w->metric, w->nharm, nv, slot_cnt);
             e = cudaGetLastError();
         }
-        listp = order;
+        /* every slot's records in trial order; invalid records (all-ones key) last */
+        cub::DoubleBuffer<uint64_t> kb(w->key[0], w->key[1]);
+        cub::DoubleBuffer<unsigned> ib(w->idx[0], w->idx[1]);
+        size_t tb = w->temp_bytes;
+        if (e == cudaSuccess)
+            e = cub::DeviceRadixSort::SortPairs(w->temp, tb, kb, ib, (int)n, 0, end_bit, st);
+        /* merged into stable r order (remove) or stable frequency order */
+        if (e == cudaSuccess) {
+            cl::slot_starts_kernel<<<1, 1, 0, st>>>(slot_cnt, nslot, slot_start);
+            cl::merge_kernel<<<g, cl::NT, 0, st>>>(ib.Current(), nv, w->slot_of, w->bkey,
+                                                   remove ? w->r : w->freq, slot_start, slot_cnt,
+                                                   nslot, w->merged);
+            e = cudaGetLastError();
+        }
+        if (remove) {
+            if (e == cudaSuccess) {
+                cl::run_flags_kernel<<<g, cl::NT, 0, st>>>(w->merged, w->r, n, nv, dr_tol, w->flag);
+                e = cudaGetLastError();
+            }
+            if (e == cudaSuccess) {
+                tb = w->temp_bytes;
+                e = cub::DeviceScan::ExclusiveSum(w->temp, tb, w->flag, w->runid, (int)n, st);
+            }
+            /* the key buffers are free once the merge has run: best-of-run slots */
+            unsigned long long *best = reinterpret_cast<unsigned long long *>(w->key[0]);
+            if (e == cudaSuccess) e = cudaMemsetAsync(best, 0, (size_t)n * sizeof(uint64_t), st);
+            if (e == cudaSuccess) {
+                cl::count_runs_kernel<<<1, 1, 0, st>>>(w->flag, w->runid, n, m);
+                cl::run_offer_kernel<<<g, cl::NT, 0, st>>>(w->merged, w->metric, w->flag, w->runid,
+                                                           nv, best);
+                cl::run_take_kernel<<<g, cl::NT, 0, st>>>(w->merged, best, n, m, w->list);
+                e = cudaGetLastError();
+            }
+        } else {
+            if (e == cudaSuccess) {
+                cl::copy_count_kernel<<<1, 1, 0, st>>>(nv, m);
+                e = cudaGetLastError();
+            }
+            list = w->merged;
+        }
     }
-    if (e == cudaSuccess) e = finish_prepare();
     if (e == cudaSuccess) {
         cl::finish_kernel<<<1, cl::FT, sizeof(cl::FinishSmem), st>>>(
-            listp, m, harm_remove, numharm, harm_tol, w->r, w->freq, w->metric, w->nharm, w->mpos,
-            w->removed, w->keep, w->out, nout);
+            list, binned ? bn.best : nullptr, binned ? bn.idx : nullptr, m, harm_remove, numharm,
+            harm_tol, w->r, w->freq, w->metric, w->nharm, w->mpos, w->removed, w->keep, w->out,
+            w->s_out, w->h_counters);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(w->h_counters, w->counters, 4 * sizeof(unsigned),
-                            cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) {
         fprintf(stderr, "Error: candidate collapse on the GPU: %s\n", cudaGetErrorString(e));
         return -1;
@@ -896,8 +1106,9 @@ int cs_collapse_finish(CsCollapse *w, cudaStream_t st, CandidateList *out)
         return 0;
     }
     {
-        const unsigned nout = w->h_counters[2];
-        if (nout > w->h_out_cap) {
+        const unsigned nout = w->h_counters[0];
+        const bool pinned = nout <= cl::CAP;
+        if (!pinned && nout > w->h_out_cap) {
             if (w->h_out) cudaFreeHost(w->h_out);
             w->h_out = nullptr;
             w->h_out_cap = 0;
@@ -906,14 +1117,16 @@ int cs_collapse_finish(CsCollapse *w, cudaStream_t st, CandidateList *out)
             if (e != cudaSuccess) goto fail;
             w->h_out_cap = nout + nout / 4 + 256;
         }
-        if (nout) {
+        if (!pinned) {
             e = cudaMemcpyAsync(w->h_out, w->out, (size_t)nout * sizeof(Candidate),
                                 cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) goto fail;
+        }
+        if (nout) {
             out->v = (Candidate *)malloc((size_t)nout * sizeof(Candidate));
             if (!out->v) return -1;
-            memcpy(out->v, w->h_out, (size_t)nout * sizeof(Candidate));
+            memcpy(out->v, pinned ? w->s_out : w->h_out, (size_t)nout * sizeof(Candidate));
             out->n = nout;
             out->cap = nout;
         }
