@@ -47,6 +47,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -194,16 +195,21 @@ __global__ void copy_count_kernel(const unsigned *src, unsigned *dst)
     *dst = *src;
 }
 
-static __device__ bool related(double r1, double r2, int numharm, double tol)
+/* whether the mm-th harmonic of the one is some harmonic of the other */
+static __device__ __forceinline__ bool related_at(double r1, double r2, int mm, int numharm, double tol)
 {
     const double lo = r1 < r2 ? r1 : r2;
     const double hi = r1 < r2 ? r2 : r1;
     if (!(lo > 0.0)) return false;
-    for (int mm = 1; mm <= numharm; mm++) {
-        const int nn = (int)rint((double)mm * hi / lo);
-        if (nn < 1 || nn > numharm) continue;
-        if (fabs((double)mm * hi - (double)nn * lo) <= tol * (double)mm) return true;
-    }
+    const int nn = (int)rint((double)mm * hi / lo);
+    if (nn < 1 || nn > numharm) return false;
+    return fabs((double)mm * hi - (double)nn * lo) <= tol * (double)mm;
+}
+
+static __device__ bool related(double r1, double r2, int numharm, double tol)
+{
+    for (int mm = 1; mm <= numharm; mm++)
+        if (related_at(r1, r2, mm, numharm, tol)) return true;
     return false;
 }
 
@@ -285,8 +291,13 @@ static __device__ void harmonics_keep(FinishShared &f, MetricSort::TempStorage &
     for (unsigned i = 0; i < m; i++) {
         if (f.rm[i]) continue;                  /* the same value in every thread */
         const double ri = f.rs[i];
-        for (unsigned j = i + 1 + tid; j < m; j += FT)
-            if (!f.rm[j] && related(f.rs[j], ri, numharm, tol)) f.rm[j] = 1;
+        /* a thread for each (candidate, harmonic): a step is one FP64 division
+         * deep, not numharm of them (40 candidates, 4 kept: 20 k cycles -> 8 k) */
+        const unsigned nh = numharm > 0 ? (unsigned)numharm : 0u, pairs = (m - i - 1) * nh;
+        for (unsigned q = tid; q < pairs; q += FT) {
+            const unsigned d = q / nh, j = i + 1 + d;
+            if (!f.rm[j] && related_at(f.rs[j], ri, (int)(q - d * nh) + 1, numharm, tol)) f.rm[j] = 1;
+        }
         __syncthreads();
     }
     for (unsigned q = tid; q < m; q += FT) f.keep[f.pos[q]] = !f.rm[q];
@@ -545,8 +556,9 @@ __global__ void __launch_bounds__(FT) finish_kernel(unsigned *list, const unsign
  * about twenty, none of which has work for more than a CTA then.  It reads the
  * record count on the device, so it can be queued behind a search whose count
  * the host does not know yet, and writes the list to pinned host memory: one
- * wait in all.  (1 M points, 300 records: 33 us of kernel against 75 us of
- * kernels, two waits and a copy; a whole pass 523 -> 428 us.) */
+ * wait in all.  (1 M points, 2000 records: 14 us of kernel, 33 with the records
+ * sorted, against 75 us of kernels, two waits and a copy; a whole pass 523 -> 428
+ * -> 410 us.) */
 template <unsigned IT>
 using SlotSort = cub::BlockRadixSort<uint32_t, FT, IT, uint16_t>;
 
@@ -563,8 +575,25 @@ struct SmallArgs {
     double r_lo, lodr, nyq, T, thr;
     int remove, harm_remove, numharm;
     double drtol, tol;
+    double inv;                     /* bins per unit of r; negative: order the records instead */
     Candidate *out;                 /* pinned, CAP */
     unsigned *status;               /* pinned: records, error flag, list length, done */
+};
+
+/* The bins of a short list, in a hash table: a bin takes a place when its first
+ * record comes.  All ones before. */
+constexpr unsigned HS = 5120;           /* places; at most CAP are taken */
+constexpr unsigned RUNS = FT;           /* runs that are ranked by counting */
+struct Hashed {
+    uint32_t key[HS];               /* bin */
+    uint32_t nmet[HS];              /* inverted order of the largest metric */
+    uint32_t qlo[HS], nqhi[HS];     /* smallest place in the bin, inverted largest */
+    uint16_t bi[HS];                /* first record of largest metric */
+    uint16_t li[HS], hi[HS];        /* records of smallest (later the run) and largest r */
+    uint16_t occ[CAP];              /* taken places */
+    uint32_t sbin[RUNS], order[RUNS];   /* bins where a run starts, as found and in order */
+    unsigned long long best[RUNS];
+    unsigned nocc, nstart;
 };
 
 struct SmallSmem {
@@ -588,10 +617,180 @@ struct SmallSmem {
             } u;
             typename cub::BlockScan<unsigned, FT>::TempStorage scan;
         } o;
+        Hashed h;
         FinishSmem fin;             /* once the list is made */
     };
 };
+static_assert(offsetof(Hashed, occ) % 16 == 0, "cleared in 16-byte stores");
 static_assert(sizeof(SmallSmem) <= 220 * 1024 && CAP == 4 * FT, "one CTA's shared memory");
+
+static __device__ __forceinline__ unsigned hash_place(uint32_t b)
+{
+    return __umulhi(b * 2654435761u, HS);
+}
+
+static __device__ __forceinline__ unsigned hash_find(const Hashed &h, uint32_t b)
+{
+    for (unsigned s = hash_place(b);; s = s + 1 == HS ? 0 : s + 1) {
+        const uint32_t k = h.key[s];
+        if (k == b) return s;
+        if (k == NONE) return NONE;
+    }
+}
+
+/* slot = i where wins(i, the record there) */
+template <class Wins>
+static __device__ __forceinline__ void offer16(uint16_t *slot, unsigned i, Wins wins)
+{
+    unsigned short old = *(volatile uint16_t *)slot;
+    while (old == 0xFFFF || wins(i, (unsigned)old)) {
+        const unsigned short was = atomicCAS((unsigned short *)slot, old, (unsigned short)i);
+        if (was == old) break;
+        old = was;
+    }
+}
+
+/* Harvest and remove_duplicates of n <= CAP records by bins (above): sm.list and
+ * sm.m, or false when there are more than RUNS runs.  A run is often hundreds of
+ * records (a strong line at every trial and decimation around it), so few bins are
+ * ordered where the sort orders all records: 2000 records in 19 runs, 40 k cycles
+ * by sort and merge, 15 k so.  What the bins need exactly (the earliest of equal metrics, the
+ * r at a bin's ends) is found in two steps, 32-bit atomics first and comparisons
+ * between the few that tie. */
+static __device__ bool hash_list(SmallSmem &sm, const SmallArgs &a, unsigned n)
+{
+    Hashed &h = sm.h;
+    const unsigned tid = threadIdx.x;
+    for (unsigned i = tid; i < offsetof(Hashed, occ) / 16; i += FT)
+        reinterpret_cast<uint4 *>(&h)[i] = make_uint4(NONE, NONE, NONE, NONE);
+    h.best[tid] = 0;
+    if (tid == 0) h.nocc = h.nstart = 0;
+    __syncthreads();
+    unsigned place[CAP / FT];
+    uint32_t nm[CAP / FT], q[CAP / FT];
+#pragma unroll
+    for (unsigned u = 0; u < CAP / FT; u++) {
+        place[u] = NONE;
+        nm[u] = q[u] = 0;
+        if (u * FT >= n) continue;
+        const unsigned i = u * FT + tid;
+        if (i < n) {
+            const CsRec rc = a.recs[i];
+            bool ok = (double)rc.metric > a.thr && rc.slot >= 0 && rc.slot < a.nslot;
+            double x = 0.0;
+            if (ok) {
+                const double rstart = a.r_lo + (double)a.chunks[rc.chunk].i0 * a.lodr;
+                const double rfreq = rstart + (double)rc.j * a.lodr;
+                const double kmul = (double)a.si.k[rc.slot];
+                x = kmul != 1.0 ? kmul * rfreq : rfreq;
+                ok = rc.slot == 0 || x < a.nyq;
+            }
+            if (ok) {
+                sm.rr[i] = x;
+                sm.met[i] = rc.metric;
+                sm.chunk[i] = rc.chunk;
+                sm.slot[i] = (unsigned char)rc.slot;
+                const double p = x * a.inv;
+                const uint32_t b = (uint32_t)p;
+                nm[u] = ~ordered_bits(rc.metric + 0.0f);
+                q[u] = (uint32_t)((p - (double)b) * 4294967296.0);
+                for (unsigned s = hash_place(b);; s = s + 1 == HS ? 0 : s + 1) {
+                    uint32_t k = *(volatile uint32_t *)&h.key[s];
+                    if (k == NONE) {
+                        k = atomicCAS(&h.key[s], NONE, b);
+                        if (k == NONE) {
+                            h.occ[atomicAdd(&h.nocc, 1u)] = (uint16_t)s;
+                            k = b;
+                        }
+                    }
+                    if (k == b) {
+                        place[u] = s;
+                        break;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        int same;
+        __match_all_sync(0xffffffffu, place[u], &same);
+        if (same) {                         /* neighbours in the list often share a bin */
+            const uint32_t m0 = __reduce_min_sync(0xffffffffu, nm[u]);
+            const uint32_t l0 = __reduce_min_sync(0xffffffffu, q[u]);
+            const uint32_t h0 = __reduce_min_sync(0xffffffffu, ~q[u]);
+            if (place[u] != NONE && (tid & 31) == 0) {
+                atomicMin(&h.nmet[place[u]], m0);
+                atomicMin(&h.qlo[place[u]], l0);
+                atomicMin(&h.nqhi[place[u]], h0);
+            }
+        } else if (place[u] != NONE) {
+            atomicMin(&h.nmet[place[u]], nm[u]);
+            atomicMin(&h.qlo[place[u]], q[u]);
+            atomicMin(&h.nqhi[place[u]], ~q[u]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (unsigned u = 0; u < CAP / FT; u++) {
+        const unsigned s = place[u], i = u * FT + tid;
+        if (s == NONE) continue;
+        if (h.nmet[s] == nm[u])
+            offer16(&h.bi[s], i, [&](unsigned y, unsigned o) {
+                if (sm.rr[y] != sm.rr[o]) return sm.rr[y] < sm.rr[o];
+                return sm.chunk[y] < sm.chunk[o] ||
+                       (sm.chunk[y] == sm.chunk[o] && sm.slot[y] < sm.slot[o]);
+            });
+        if (h.qlo[s] == q[u])
+            offer16(&h.li[s], i, [&](unsigned y, unsigned o) { return sm.rr[y] < sm.rr[o]; });
+        if (h.nqhi[s] == ~q[u])
+            offer16(&h.hi[s], i, [&](unsigned y, unsigned o) { return sm.rr[y] > sm.rr[o]; });
+    }
+    __syncthreads();
+    const unsigned nocc = h.nocc;
+    for (unsigned o = tid; o < nocc; o += FT) {
+        const unsigned s = h.occ[o];
+        const uint32_t b = h.key[s];
+        unsigned p = b >= 1 ? hash_find(h, b - 1) : NONE;
+        if (p == NONE && b >= 2) p = hash_find(h, b - 2);
+        if (p == NONE || sm.rr[h.li[s]] - sm.rr[h.hi[p]] > a.drtol) {
+            const unsigned at = atomicAdd(&h.nstart, 1u);
+            if (at < RUNS) h.sbin[at] = b;
+        }
+    }
+    __syncthreads();
+    const unsigned m = h.nstart;
+    if (m > RUNS) return false;
+    if (tid < m) {
+        const uint32_t b = h.sbin[tid];
+        unsigned rank = 0;
+#pragma unroll 4
+        for (unsigned i = 0; i < m; i++) rank += h.sbin[i] < b ? 1u : 0u;
+        h.order[rank] = b;
+    }
+    __syncthreads();
+    for (unsigned o = tid; o < nocc; o += FT) {
+        const unsigned s = h.occ[o];
+        const uint32_t b = h.key[s];
+        unsigned lo = 0, e = m;             /* the last start at or before b */
+        while (e - lo > 1) {
+            const unsigned mid = (lo + e) >> 1;
+            if (h.order[mid] <= b) lo = mid;
+            else e = mid;
+        }
+        h.li[s] = (uint16_t)lo;
+        atomicMax(&h.best[lo], ((unsigned long long)~h.nmet[s] << 32) |
+                                   (unsigned long long)(0xFFFFFFFFu - b));
+    }
+    __syncthreads();
+    for (unsigned o = tid; o < nocc; o += FT) {
+        const unsigned s = h.occ[o];
+        const unsigned long long key = ((unsigned long long)~h.nmet[s] << 32) |
+                                       (unsigned long long)(0xFFFFFFFFu - h.key[s]);
+        if (h.best[h.li[s]] == key) sm.list[h.li[s]] = h.bi[s];
+    }
+    if (tid == 0) sm.m = m;
+    __syncthreads();
+    return true;
+}
 
 /* Harvest, order and remove_duplicates of n <= IT * FT records: sm.list, sm.m. */
 template <unsigned IT>
@@ -715,9 +914,11 @@ __global__ void __launch_bounds__(FT) collapse_small(const __grid_constant__ Sma
         a.status[3] = err == 0 && n <= a.cap && n <= CAP ? 1u : 0u;
     }
     if (err != 0 || n > a.cap || n > CAP || n == 0) return;
-    if (n <= FT) small_list<1>(sm, a, n, sm.o.u.sort1);
-    else if (n <= 2 * FT) small_list<2>(sm, a, n, sm.o.u.sort2);
-    else small_list<4>(sm, a, n, sm.o.u.sort4);
+    if (a.inv < 0.0 || !hash_list(sm, a, n)) {
+        if (n <= FT) small_list<1>(sm, a, n, sm.o.u.sort1);
+        else if (n <= 2 * FT) small_list<2>(sm, a, n, sm.o.u.sort2);
+        else small_list<4>(sm, a, n, sm.o.u.sort4);
+    }
     const unsigned m = sm.m;
     if (a.harm_remove)
         harmonics_keep(sm.fin.f, sm.fin.t.sort, m, a.numharm, a.tol,
@@ -882,6 +1083,24 @@ static int bit_length_u64(uint64_t v)
     return b;
 }
 
+/* Bins along r for a search's trials; inv is negative where they do not hold.
+ * They are a millionth narrower than dr_tol; rounding of r and of its product
+ * with inv stays below that for up to 2^27 of them.  r >= 0 keeps the order of
+ * the bits. */
+struct BinScale {
+    double inv, bins;
+};
+
+static BinScale bin_scale(double r_lo, double lodr, double trials, int k0, double N, double dr_tol)
+{
+    BinScale s = {-1.0, 0.0};
+    if (!(dr_tol > 0.0) || !(r_lo >= 0.0) || !(lodr > 0.0)) return s;
+    const double width = dr_tol * (1.0 - 1e-6);
+    s.bins = std::max(N / 2.0, (r_lo + trials * lodr) * (double)k0) / width + 2.0;
+    if (s.bins < (double)(1 << 27)) s.inv = 1.0 / width;
+    return s;
+}
+
 int cs_collapse_small_enqueue(CsCollapse *w, const CsRec *recs, const unsigned *count,
                               const int *err, unsigned cap, const CsChunk *chunks,
                               const int *slot_k, const int *slot_Hk, int nslot, long long total,
@@ -912,6 +1131,7 @@ int cs_collapse_small_enqueue(CsCollapse *w, const CsRec *recs, const unsigned *
     a.numharm = numharm;
     a.drtol = dr_tol;
     a.tol = harm_tol;
+    a.inv = remove ? bin_scale(r_lo, lodr, (double)total, slot_k[0], N, dr_tol).inv : -1.0;
     a.out = w->s_out;
     a.status = w->s_status;
     w->s_status[3] = 0;
@@ -945,24 +1165,17 @@ int cs_collapse_small_status(const CsCollapse *w, unsigned *n, int *err)
  * and its list some 20 launches.  Sort against bins, with both waits: 5 k records
  * in 0.1, 0.5 and 4.2 M bins 156:78, 166:96 and 194:147 us, 80 k records in the
  * same 267:105, 345:222 and 662:564.  The ends would meet near 2 k bins a record;
- * BINS_MOST bounds the memory (336 MB).
- * They are a millionth narrower than dr_tol; rounding of r and of its product
- * with inv stays below that for up to 2^27 of them.  r >= 0 keeps the
- * order of the bits. */
+ * BINS_MOST bounds the memory (336 MB). */
 static bool bins_for(CsCollapse *w, unsigned n, long long nchunks, const cl::SlotInfo &si,
                      int nprof, double r_lo, double lodr, double N, double dr_tol, cudaStream_t st,
                      cl::Bins &bn)
 {
-    if (!(dr_tol > 0.0) || !(r_lo >= 0.0) || !(lodr > 0.0)) return false;
-    const double width = dr_tol * (1.0 - 1e-6);
-    const double top = std::max(
-        N / 2.0, (r_lo + (double)nchunks * (double)nprof * lodr) * (double)si.k[0]);
-    const double want = top / width + 2.0;
+    const BinScale sc = bin_scale(r_lo, lodr, (double)nchunks * (double)nprof, si.k[0], N, dr_tol);
     const unsigned long long most =
         std::min((unsigned long long)n * cl::BINS_PER_REC, cl::BINS_MOST);
-    if (!(want < (double)most)) return false;
-    bn.nb = (unsigned)want;
-    bn.inv = 1.0 / width;
+    if (!(sc.inv >= 0.0) || !(sc.bins < (double)most)) return false;
+    bn.nb = (unsigned)sc.bins;
+    bn.inv = sc.inv;
     const size_t pad = ((size_t)bn.nb + cl::BT - 1) / cl::BT * cl::BT, blocks = pad / cl::BT;
     const size_t ones = ((size_t)n + 2 * (size_t)bn.nb) * sizeof(uint64_t) + (size_t)bn.nb * 4;
     const size_t bytes = ones + pad / 8 + blocks * 4;
