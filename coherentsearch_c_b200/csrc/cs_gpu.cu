@@ -1197,11 +1197,11 @@ static void cols_launch(int nh, int grid, int smem, cudaStream_t st, const wsk::
                         const cols::XArgs &x)
 {
     if (nh == 60)
-        cols::search_cols<wsk::Cfg60><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+        cols::search_cols<wsk::Cfg60><<<grid, cols::Roles<wsk::Cfg60>::NTHREADS, smem, st>>>(w, x);
     else if (nh == 32)
-        cols::search_cols<wsk::Cfg32><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+        cols::search_cols<wsk::Cfg32><<<grid, cols::Roles<wsk::Cfg32>::NTHREADS, smem, st>>>(w, x);
     else
-        cols::search_cols<wsk::Cfg16><<<grid, cols::NTHREADS, smem, st>>>(w, x);
+        cols::search_cols<wsk::Cfg16><<<grid, cols::Roles<wsk::Cfg16>::NTHREADS, smem, st>>>(w, x);
 }
 
 /* The geometry of the register-block kernel: columns D trials apart (the

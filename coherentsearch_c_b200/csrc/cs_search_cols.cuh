@@ -21,10 +21,11 @@
  * the reference's 16 fused multiply-adds in tap order (adding 0 * x between
  * them changes nothing for finite x).
  *
- * Measured: 8.05 M trials at nharms 60 4.68 -> 2.53 ms, 3.0 M at 32 0.474 ->
- * 0.34, 1.1 M at 16 0.219 -> 0.174.  What bounds it now is the interpolation
- * warps (half their time in the multiply-adds, whose shared-memory reads keep
- * that path 55 % busy over the kernel; issue slots 60 %).
+ * Measured: 8.05 M trials at nharms 60 4.68 -> 2.31 ms, 1.0 M 0.70 -> 0.336, 3.0 M
+ * at 32 0.474 -> 0.331, 1.1 M at 16 0.219 -> 0.152.  No unit is full (issue slots
+ * 63 % busy, 70 % on the fullest scheduler; shared-memory path 47 %, FP32 44 %): the
+ * ring of window stages is what binds, a third of an interpolation warp's time
+ * going into waits for boxes at nharms 60; at 32 and 16 the epilogue is as long.
  *
  *   tile      128 trials: 16 consecutive (a phase block) x 8 columns;
  *             row (k * 4 + j) * 8 + cg * 4 + g is trial 4g + k of the phase
@@ -36,11 +37,11 @@
  *   windows   a padded copy of the spectrum (pad_amax_kernel); per (tile,
  *             harmonic) one TMA box of 8 rows (the columns, a fixed number of
  *             bins apart) into a ring of stages, four harmonics a stage.
- *   warps     0-3 interpolate (a stage each in turn: 4 harmonics x 8 threads)
- *             into a shared-memory ring of A operand K steps; 4-11 run the
- *             boxcar epilogue from tensor memory; 12 and 13 issue the TMA
- *             boxes; 14 finds each row's chunk; 15 copies each K step (8
- *             harmonics) to tensor memory on arrival and issues the MMAs.
+ *   warps     8 (nharms 16: 4) interpolate (a stage each in turn: 4 harmonics x
+ *             8 threads) into a shared-memory ring of A operand K steps; 8 run
+ *             the boxcar epilogue from tensor memory; 2 issue the TMA boxes; one
+ *             finds each row's chunk; one copies each K step (8 harmonics) to
+ *             tensor memory on arrival and issues the MMAs.
  *
  * Every wait is bounded; one that gives up sets the session's error flag and
  * a CTA-wide one that the other roles see, copies and MMAs in flight are
@@ -53,10 +54,20 @@ namespace cols {
 using wsk::Args;
 using wsk::TMEM_COLS;
 
-constexpr int NTHREADS = 16 * 32;
-constexpr int NINT = 4, NEPI = 8;             /* interpolation, epilogue warps */
+constexpr int NEPI = 8;                       /* epilogue warps */
 constexpr int NTMA = 2;                       /* warps that issue the boxes */
-constexpr int WARP_TMA = NINT + NEPI, WARP_ROW = WARP_TMA + NTMA, WARP_MMA = WARP_ROW + 1;
+/* The warps of a configuration: interpolation, epilogue, boxes, rows, MMA.  One
+ * interpolation warp a scheduler waits for its own loads, rotations and stores
+ * (1 M trials at nharms 60: 361 us); two of them hide that (341), with registers
+ * moved from the other roles: 640 x 96 are launched, 8 x 32 x 120 + 8 x 32 x 88 +
+ * 4 x 32 x 64 are used, the same sum.  Four warps on the boxes would leave 112 and
+ * 80: slower (364).  nharms 16 has 4 blocks a tile, one a warp. */
+template <class C>
+struct Roles {
+    static constexpr int NINT = C::NH >= 32 ? 8 : 4;
+    static constexpr int TMA = NINT + NEPI, ROW = TMA + NTMA, MMA = ROW + 1;
+    static constexpr int NTHREADS = 32 * (MMA + 1);
+};
 constexpr int TI = 16, TC = 8;                /* consecutive trials, columns of a tile */
 /* tensor memory: NACC accumulators, then NAB copies of a tile's A operand (hi:
  * K/2 columns, then lo) */
@@ -67,12 +78,12 @@ struct Tm {
 };
 constexpr int MAX_ACC = 6;
 constexpr int NROW = 4;                       /* row-info slots */
-constexpr int NA = 4;                         /* A operand K steps in the ring */
+/* A operand K steps in the ring.  A warp's block before this one was at most 5
+ * steps back, so its slot's use two back is complete: a parity needs that. */
+constexpr int NA = 5;
 constexpr int A_STEP = 2 * 2 * CS_TILE_M * 16;    /* bytes: hi and lo, two K blocks each */
 constexpr int MAX_STG = 10;                   /* most window stages */
-/* fewest: the A ring lets a warp run at most 11 blocks ahead of another, less
- * than two uses of a stage */
-constexpr int MIN_STG = 6;
+constexpr int MIN_STG = 4;                    /* fewest */
 constexpr int FRONT = 16;                     /* zero bins before the padded copy */
 
 /* Per phase block, contiguous in global and shared memory:
@@ -134,6 +145,28 @@ static __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity,
         if (mbar_try(bar, parity)) return true;
         if ((n & 15) == 0 && (*stop || global_ns() - t0 > CS_WAIT_NS)) return false;
     }
+}
+
+/* The same for a count in shared memory to reach n. */
+static __device__ __forceinline__ bool count_wait(const volatile int *count, int n,
+                                                  const volatile int *stop)
+{
+    if (*count >= n) return true;
+    const unsigned long long t0 = global_ns();
+    for (int i = 1;; i++) {
+        if (*count >= n) return true;
+        if ((i & 15) == 0 && (*stop || global_ns() - t0 > CS_WAIT_NS)) return false;
+    }
+}
+
+/* One lane of the warp, known to the compiler as one: what it issues takes its
+ * operands from uniform registers without a loop over lanes. */
+static __device__ __forceinline__ bool elect()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
 static __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes)
@@ -547,9 +580,10 @@ static __device__ __forceinline__ void store_rows(const float2 (&acc)[4][4], flo
 }
 
 template <class C>
-__global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant__ Args a,
+__global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __grid_constant__ Args a,
                                                            const __grid_constant__ XArgs x)
 {
+    constexpr int NINT = Roles<C>::NINT, WARP_TMA = Roles<C>::TMA, WARP_ROW = Roles<C>::ROW;
     constexpr int NPAD = C::NPAD, NBLK = C::NH / 4, NKS = (NBLK + 1) / 2;
     constexpr unsigned long long ALL = C::NH == 64 ? ~0ull : (1ull << C::NH) - 1;
     static_assert(NBLK >= NINT, "every interpolation warp has a block in every tile");
@@ -566,7 +600,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
                    bbar = tbar + 8;
     volatile int *stop = reinterpret_cast<volatile int *>(smem + L.bar + 496);
     uint32_t *tm_slot = reinterpret_cast<uint32_t *>(smem + L.bar + 500);
-    static_assert(8 * (2 * MAX_STG + 2 * NA + 2 * MAX_ACC + 2 * NROW + 2) <= 496, "barriers");
+    static_assert(8 * (2 * MAX_STG + 2 * NA + 2 * MAX_ACC + 2 * NROW + 2) <= 448, "barriers");
+    /* uses of each window stage that its reader has begun with */
+    volatile int *used = reinterpret_cast<volatile int *>(smem + L.bar + 448);
     static_assert(NACC >= 3 && NACC <= MAX_ACC, "the epilogue holds two accumulators");
     unsigned long long *row_fill = reinterpret_cast<unsigned long long *>(smem + L.row);
     int *row_ci = reinterpret_cast<int *>(smem + L.row + NROW * CS_TILE_M * 8);
@@ -597,6 +633,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
         }
         mbar_init(tbar, 1);
         mbar_init(bbar, 1);
+        for (int i = 0; i < MAX_STG; i++) used[i] = 0;
         *stop = 0;
         /* the B images, behind the other set-up; the MMA warp waits for them */
         fence_proxy_async();
@@ -635,6 +672,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
         return wait_bar(b + 8 * slot, use & 1, stop);
     };
 
+    if constexpr (NINT == 8) {      /* by groups of 4 warps, all through here */
+        if (warp < NINT) asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        else if (warp < WARP_TMA) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    }
     if (warp < NINT) {
         /* ------------------------- interpolation ------------------------- */
         const int hh = lane >> 3, cg = (lane >> 2) & 1, gr = lane & 3;
@@ -643,7 +685,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
         const int nunit = nt * NBLK;
         int it = -1, itn = 0, hb = warp, all = 1, pb = tb / g.ncg - 1, loads = 0;
         int pb_end = tb;                     /* first tile past phase block pb */
-        int st = warp, round = 0;       /* nstg > NINT */
+        int st = warp % g.nstg, round = warp / g.nstg;
         bool ok = true;
         /* what a block needs from shared memory is read while the block before
          * is stored: its rows' shape, and the groups' window offsets */
@@ -671,8 +713,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
             const int ks = it * NKS + (hb >> 1), as = ks % NA;
             /* the stage's last use first: its reader may be another warp that is
              * behind, and a parity says nothing about a phase two back */
-            if (round > 0) ok = full_wait(wempty, st, round - 1) && ok;
+            ok = count_wait(used + st, round, stop) && ok;
             ok = full_wait(wfull, st, round) && ok;
+            if (lane == 0) used[st] = round + 1;
             const bool afree = ks < NA || mbar_try(aempty + 8 * as, (ks / NA - 1) & 1);
             const float4 *gp = reinterpret_cast<const float4 *>(tab + g.g_off) + h * 8 + 2 * gr;
             float4 gn[2] = {gp[0], gp[1]};
@@ -696,7 +739,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
                 itn++;
             }
             st += NINT;
-            if (st >= g.nstg) {
+            while (st >= g.nstg) {
                 st -= g.nstg;
                 round++;
             }
@@ -785,11 +828,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
         int p = tb / g.ncg, cgi = tb - p * g.ncg;
         int n = 0, st = 0, round = 0;
         bool ok = true;
-        const int hl = 2 * me + (lane & 1);      /* of the block */
+        /* a lane holds what its box of the tile needs, block lane / 2: nothing is
+         * computed or read between a stage's wait and its boxes (the two warps
+         * were busy all the time: 1 M trials 341 -> 336 us, 1.1 M at nharms 16 174 ->
+         * 152) */
+        const int mine = lane >> 1, hl = 4 * min(mine, NBLK - 1) + 2 * me + (lane & 1);
         const int *x0 = reinterpret_cast<const int *>(smem + L.tab + g.x_off);
-        const char *maps = reinterpret_cast<const char *>(x.maps) + hl * 128;
+        const char *maps = reinterpret_cast<const char *>(x.maps) + 2 * me * 128;
+        const int pitch = blk[min(mine, NBLK - 1)].y;
         const uint32_t dst = sbase + L.win;
-        const int s1 = g.shift[0];               /* a column's bins, per harmonic number */
+        const int step = 2 * TC * g.shift[0] * (hl + 1);     /* floats a column group */
+        int xp = 0;
         for (int it = 0; it < nt && ok; it++) {
             if (p != pb) {
                 pb = p;
@@ -808,27 +857,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) search_cols(const __grid_constant
                     __syncwarp();
                 }
                 ok = full_wait(tbar, 0, loads++) && ok;
+                xp = 2 * x0[hl];
             }
-            /* the next block's numbers are read behind this one's wait */
-            int xn = x0[hl], pn = blk[0].y;
+            /* a multiple of 4 floats: the box starts on 16 bytes */
+            const int xc = (xp + cgi * step) & ~3;
+#pragma unroll 1
             for (int hb = 0; hb < NBLK; hb++, n++) {
-                const int pitch = pn, h1 = 4 * hb + hl + 1;
-                /* a multiple of 4 floats: the box starts on 16 bytes */
-                const int xc = 2 * (xn + cgi * (TC * s1) * h1) & ~3;
-                if (hb + 1 < NBLK) {
-                    xn = x0[4 + h1 - 1];
-                    pn = blk[hb + 1].y;
-                }
                 if (round > 0) ok = full_wait(wempty, st, round - 1) && ok;
                 if (__any_sync(0xffffffffu, !ok)) {
                     ok = false;
                     break;
                 }
-                if (lane == 0) expect_tx(wfull + 8 * st, (uint32_t)(2 * TC * pitch));
+                const int xa = __shfl_sync(0xffffffffu, xc, 2 * hb);
+                const int xb = __shfl_sync(0xffffffffu, xc, 2 * hb + 1);
+                const uint32_t rows = __shfl_sync(0xffffffffu, (uint32_t)(TC * pitch), 2 * hb);
+                const uint32_t b = wfull + 8 * st, to = dst + st * g.stg_bytes + 2 * me * rows;
+                const char *m = maps + hb * 512;
+                if (elect()) {
+                    expect_tx(b, 2 * rows);
+                    tma_rows(to, m, xa, b);
+                    tma_rows(to + rows, m + 128, xb, b);
+                }
                 __syncwarp();
-                if (lane < 2)
-                    tma_rows(dst + st * g.stg_bytes + hl * TC * pitch, maps + hb * 512, xc,
-                             wfull + 8 * st);
                 if (++st == g.nstg) {
                     st = 0;
                     round++;
