@@ -55,7 +55,7 @@ DFT_FLOP_PER_TRIAL = 28560.0      # 2*(2nh-1)*2nh at nh=60 (k | nh folds add non
 SIMT_OPS_PER_TRIAL = 6000.0       # interp 1920 FMA + 360 rotate + boxcar/fold ~3700
 
 
-KERNEL_NAMES = {0: "cs_search_kernel", 1: "search_ws_cfg60", 2: "search_f64",
+KERNEL_NAMES = {0: "cs_search_kernel", 1: "search_cols_cfg60", 2: "search_f64",
                 3: "search_tma_cfg60", 4: "interp_tc + search_pre_cfg60"}
 
 
@@ -963,7 +963,7 @@ def run_prep(args):
         "gpu_launches": (8 + 16 * t.ndm) * args.steps,
         "roofline": {"bound": "tensor", "achieved": dft_tflops, "peak": tc_peak,
                      "unit": "TFLOP/s", "frac": dft_tflops / tc_peak, "traffic": None,
-                     "kernel": "search_ws_cfg60", "kernel_ms_per_dm": kms / t.ndm,
+                     "kernel": "search_cols_cfg60", "kernel_ms_per_dm": kms / t.ndm,
                      "peak_kind": f"bf16 dense, {peak_kind}",
                      "algorithmic": f"{DFT_FLOP_PER_TRIAL:.0f} DFT flop/trial x {total} trials "
                                     f"x {t.ndm} DMs"},

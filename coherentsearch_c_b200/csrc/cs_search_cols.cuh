@@ -23,9 +23,10 @@
  *
  * Measured: 8.05 M trials at nharms 60 4.68 -> 2.31 ms, 1.0 M 0.70 -> 0.336, 3.0 M
  * at 32 0.474 -> 0.331, 1.1 M at 16 0.219 -> 0.152.  No unit is full (issue slots
- * 63 % busy, 70 % on the fullest scheduler; shared-memory path 47 %, FP32 44 %): the
- * ring of window stages is what binds, a third of an interpolation warp's time
- * going into waits for boxes at nharms 60; at 32 and 16 the epilogue is as long.
+ * 63 % busy, 70 % on the fullest scheduler; shared-memory path 47 %, FP32 44 %): at
+ * nharms 60 a third of an interpolation warp's time goes into waits for boxes, 60
+ * small ones a tile (8 rows of some 200 bytes, 175 cycles each as it runs; 8
+ * stages or 10, 5 K steps or 6 are the same); at 32 and 16 the epilogue is as long.
  *
  *   tile      128 trials: 16 consecutive (a phase block) x 8 columns;
  *             row (k * 4 + j) * 8 + cg * 4 + g is trial 4g + k of the phase
