@@ -796,7 +796,7 @@ def dedisp_measure(args, world, rank, local, pg):
                        output_per_dm=nout, blocks_per_read=t.blocks_per_read,
                        l2="inputs larger than L2 (raw input and output both > 126 MB)",
                        parallelism=f"replicas{world}"),
-        "gpu_launches": (8 if args.clipped else 2) * args.steps,
+        "gpu_launches": (11 if args.clipped else 2) * args.steps,
         "roofline": {"bound": "hbm", "achieved": alg_bytes / (kern_ms * 1e-3) / 1e9,
                      "peak": hbm_peak, "unit": "GB/s",
                      "frac": alg_bytes / (kern_ms * 1e-3) / 1e9 / hbm_peak, "traffic": None,
@@ -958,9 +958,9 @@ def run_prep(args):
                        output_per_dm=ps.nout,
                        l2="inputs larger than L2 (raw input and dedispersed output > 126 MB)",
                        parallelism=f"replicas{world}"),
-        # clip decisions and levels 6, dedispersion 2; per DM spectrum 4, search 2,
-        # collapse 10 (cuFFT, CUB and PyTorch's fills not counted)
-        "gpu_launches": (8 + 16 * t.ndm) * args.steps,
+        # clip decisions and levels 5, dedispersion 2; per DM spectrum 3, search 2,
+        # collapse 1 (4 for a long list; cuFFT and PyTorch's fills not counted)
+        "gpu_launches": (7 + 6 * t.ndm) * args.steps,
         "roofline": {"bound": "tensor", "achieved": dft_tflops, "peak": tc_peak,
                      "unit": "TFLOP/s", "frac": dft_tflops / tc_peak, "traffic": None,
                      "kernel": "search_cols_cfg60", "kernel_ms_per_dm": kms / t.ndm,
@@ -1533,7 +1533,7 @@ def run_series(args):
                    "parallelism": "replicas1"},
         "e2e": {"value": total / (statistics.mean(e2e) * 1e-3), "unit": UNIT,
                 "h2d_bytes_per_step": int(x.nbytes), "d2h_bytes_per_step": int(out.nbytes)},
-        "gpu_launches": 16 * args.steps,     # 4 spectrum, 2 search, 10 collapse (cuFFT, CUB not counted)
+        "gpu_launches": 6 * args.steps,      # 3 spectrum, 2 search, 1 collapse (cuFFT not counted)
         "roofline": {"bound": "tensor", "achieved": dft, "peak": tc_peak, "unit": "TFLOP/s",
                      "frac": dft / tc_peak, "traffic": None,
                      "kernel": KERNEL_NAMES.get(ses.info().kernel, "unknown"),
