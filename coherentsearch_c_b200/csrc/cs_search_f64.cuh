@@ -326,22 +326,25 @@ static __device__ __forceinline__ void scan_bins(const double *P, const CsSlot &
 }
 
 /* Largest bin, largest pair of neighbours (cyclic) and total of the KC-fold
- * sums (KC 0: k-fold) of an FP32 row. */
+ * sums (KC 0: k-fold) of an FP32 row, and the largest size of its own bins. */
 template <int KC>
 static __device__ __forceinline__ void row_sums(const float *row, int nk, int k, float &m1,
-                                                float &m2, float &tot)
+                                                float &m2, float &tot, float &size)
 {
     const int K = KC ? KC : k;
     float last = -INFINITY, first = 0.0f;
     m1 = m2 = -INFINITY;
-    tot = 0.0f;
+    tot = size = 0.0f;
 #pragma unroll 4
     for (int j = 0; j < nk; j += 2) {           /* nk = 2 Hk is even */
         float a = row[j], b = row[j + 1];
+        size = wsk::fmax3(size, fabsf(a), fabsf(b));
 #pragma unroll
         for (int q = 1; q < K; q++) {
-            a += row[j + q * nk];
-            b += row[j + 1 + q * nk];
+            const float x = row[j + q * nk], y = row[j + 1 + q * nk];
+            size = wsk::fmax3(size, fabsf(x), fabsf(y));
+            a += x;
+            b += y;
         }
         if (j == 0) first = a;
         tot += a + b;
@@ -354,8 +357,16 @@ static __device__ __forceinline__ void row_sums(const float *row, int nk, int k,
 
 /* A bound of the FP64 metric of one profile, from its bins in FP32 (row: this
  * trial's).  As in the FP32 kernels, the largest bin and the largest pair of
- * neighbours bound every wider window; the margin is more than what the
- * roundings of either side come to. */
+ * neighbours bound every wider window.  The margin has two parts, u = 2^-24:
+ *   - a sum over the profile is at most |tot| + nk * m1 in size, and wrong by nk * u
+ *     of that;
+ *   - a folded bin is wrong by u of the K bins it was made of, each up to `size`
+ *     and rounded to FP32 before they cancel: K + K (K - 1) of u * size, or K^2.
+ *     The pairs' additions add 2 K, a window of w bins and its share of the total
+ *     have w of both: w * 2 K (K + 1) * u * size.  A tone at a harmonic that is no
+ *     multiple of K leaves a fold that small beside its bins.
+ * Where FP32 does not hold the bins (or one is no number) the answer is infinity,
+ * and what lies below its range is covered by an absolute 1e-30. */
 static __device__ __forceinline__ float slot_bound(const float *row, const CsSlot &sl,
                                                    const double *sc)
 {
@@ -365,17 +376,19 @@ static __device__ __forceinline__ float slot_bound(const float *row, const CsSlo
     for (int a = 0; a < CS_NWMAX; a++) scale[a] = a < sl.nw ? (float)sc[1 + a] : 0.0f;
     const int nk = sl.nk, K = sl.fold ? sl.k : 1;
     row += sl.fold ? 0 : sl.col0;
-    float m1, m2, tot;
+    float m1, m2, tot, size;
     switch (K) {
-    case 1: row_sums<1>(row, nk, 1, m1, m2, tot); break;
-    case 2: row_sums<2>(row, nk, 2, m1, m2, tot); break;
-    case 3: row_sums<3>(row, nk, 3, m1, m2, tot); break;
-    case 4: row_sums<4>(row, nk, 4, m1, m2, tot); break;
-    case 5: row_sums<5>(row, nk, 5, m1, m2, tot); break;
-    case 6: row_sums<6>(row, nk, 6, m1, m2, tot); break;
-    default: row_sums<0>(row, nk, K, m1, m2, tot);
+    case 1: row_sums<1>(row, nk, 1, m1, m2, tot, size); break;
+    case 2: row_sums<2>(row, nk, 2, m1, m2, tot, size); break;
+    case 3: row_sums<3>(row, nk, 3, m1, m2, tot, size); break;
+    case 4: row_sums<4>(row, nk, 4, m1, m2, tot, size); break;
+    case 5: row_sums<5>(row, nk, 5, m1, m2, tot, size); break;
+    case 6: row_sums<6>(row, nk, 6, m1, m2, tot, size); break;
+    default: row_sums<0>(row, nk, K, m1, m2, tot, size);
     }
-    const float margin = (fabsf(tot) + nk * fabsf(m1)) * (nk + 16) * 2.4e-7f;
+    if (!(size < 1e30f) || tot != tot) return INFINITY;
+    const float margin = (fabsf(tot) + nk * fabsf(m1)) * (nk + 16) * 2.4e-7f +
+                         (float)(2 * K * (K + 1) * sl.wmax) * 6.0e-8f * size + 1e-30f;
     float bound = -INFINITY;
 #pragma unroll
     for (int a = 0; a < CS_NWMAX; a++) {
