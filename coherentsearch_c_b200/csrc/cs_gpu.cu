@@ -707,6 +707,8 @@ struct GpuSession {
     unsigned char *d_cols; /* tensor maps [nh], tables, padded spectrum copy */
     size_t c_cols;
     float2 *d_pad;         /* the copy, in d_cols */
+    double thresh;         /* of the last search queued, and whether it was timed */
+    bool timed;
     CUtensorMap *h_cmaps;  /* [MAX_NH], 64-byte aligned */
     /* interpolation as tensor-core GEMMs (tci::interp_tc), then search_pre */
     int use_tci;
@@ -1778,6 +1780,8 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
                                   bool timed)
 {
     cudaError_t e;
+    S->thresh = threshold;
+    S->timed = timed;
     /* the spectrum maximum, the record count and the error flag */
     if ((e = cudaMemsetAsync(S->d_amax, 0, 4 * sizeof(unsigned), S->st)) != cudaSuccess) return e;
     if (S->namps > 0) {
@@ -1910,22 +1914,43 @@ static int collect64(GpuSession *S, unsigned n, double threshold, CandidateList 
     return 0;
 }
 
+/* Wait for the queued search; its record count to *n.  A spectrum that
+ * search_cols left alone is searched again, from the session's copy, by the
+ * kernel its geometry would have without it. */
+static int search_wait(GpuSession *S, unsigned *n)
+{
+    for (int again = 0;; again++) {
+        cudaError_t e;
+        if ((e = cudaMemcpyAsync(S->h_count, S->d_count, 2 * sizeof(unsigned),
+                                 cudaMemcpyDeviceToHost, S->st)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(S->st)) != cudaSuccess) {
+            fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
+            return -1;
+        }
+        *n = S->h_count[0];
+        if (S->h_count[1] == 0) return 0;       /* the error flag */
+        if (S->h_count[1] != cols::NOT_FINITE || !S->use_cols || again) {
+            fprintf(stderr, "Error: B200 search kernel timed out waiting for the tensor cores\n");
+            return -1;
+        }
+        const int nh = S->use_cols;
+        S->use_cols = 0;
+        e = enqueue_search(S, S->d_pad + cols::FRONT, S->thresh, S->timed);
+        S->use_cols = nh;
+        if (e != cudaSuccess) {
+            fprintf(stderr, "Error: B200 search launch failed: %s\n", cudaGetErrorString(e));
+            return -1;
+        }
+    }
+}
+
 /* Read back the records and build the candidate list. */
 static int collect(GpuSession *S, double threshold, CandidateList *out, int *need_rerun)
 {
     *need_rerun = 0;
     cudaError_t e;
-    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||       /* the count and the error flag */
-        (e = cudaStreamSynchronize(S->st)) != cudaSuccess) {
-        fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
-        return -1;
-    }
-    if (S->h_count[1] != 0) {
-        fprintf(stderr, "Error: B200 search kernel timed out waiting for the tensor cores\n");
-        return -1;
-    }
-    const unsigned n = S->h_count[0];
+    unsigned n;
+    if (search_wait(S, &n) != 0) return -1;
     if (S->prec64) return collect64(S, n, threshold, out, need_rerun);
     if (n > S->cap) {
         if (grow_records(S, n + n / 8 + 1024) != 0) return -1;
@@ -2115,18 +2140,8 @@ CS_EXPORT int cs_b200_session_collapse_enqueue(GpuSession *S, double threshold, 
                         "search with cs_b200_session_collect\n");
         return -1;
     }
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(S->h_count, S->d_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             S->st)) != cudaSuccess ||       /* the count and the error flag */
-        (e = cudaStreamSynchronize(S->st)) != cudaSuccess) {
-        fprintf(stderr, "Error: B200 search failed: %s\n", cudaGetErrorString(e));
-        return -1;
-    }
-    if (S->h_count[1] != 0) {
-        fprintf(stderr, "Error: B200 search kernel timed out waiting for the tensor cores\n");
-        return -1;
-    }
-    const unsigned n = S->h_count[0];
+    unsigned n;
+    if (search_wait(S, &n) != 0) return -1;
     if (n > S->cap) {
         if (grow_records(S, n + n / 8 + 1024) != 0) return -1;
         return 1;

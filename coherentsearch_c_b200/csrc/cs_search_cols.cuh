@@ -19,7 +19,10 @@
  * one window of NT = 18 or 20 taps that starts at an even bin; their weight
  * rows are shifted inside it and padded with zeros, which leaves each chain
  * the reference's 16 fused multiply-adds in tap order (adding 0 * x between
- * them changes nothing for finite x).
+ * them changes nothing for finite x).  A spectrum with a bin that is not finite
+ * is left alone (NOT_FINITE): 0 times such a bin would spoil trials whose own 16
+ * taps miss it.  (Skipping the padding in a second loop for such spectra cost
+ * every other one 1.5 %: the host runs the kernel for any geometry instead.)
  *
  * Measured: 8.05 M trials at nharms 60 4.68 -> 2.31 ms, 1.0 M 0.70 -> 0.336, 3.0 M
  * at 32 0.474 -> 0.331, 1.1 M at 16 0.219 -> 0.152.  No unit is full (issue slots
@@ -86,6 +89,7 @@ constexpr int A_STEP = 2 * 2 * CS_TILE_M * 16;    /* bytes: hi and lo, two K blo
 constexpr int MAX_STG = 10;                   /* most window stages */
 constexpr int MIN_STG = 4;                    /* fewest */
 constexpr int FRONT = 16;                     /* zero bins before the padded copy */
+constexpr int NOT_FINITE = 2;                 /* error flag: no tile was searched */
 
 /* Per phase block, contiguous in global and shared memory:
  *   weights   per block hb of 4 harmonics, harmonic, tap: 16 floats (trials)
@@ -612,7 +616,8 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
     int4 *blk = reinterpret_cast<int4 *>(smem + L.bar + 512);
     const int tb = (int)(((long long)g.ntiles * blockIdx.x) / gridDim.x);
     const int te = (int)(((long long)g.ntiles * (blockIdx.x + 1)) / gridDim.x);
-    const int nt = te - tb;
+    const bool finite = a.amax[1] == 0u;
+    const int nt = finite ? te - tb : 0;
 
     if (warp == 0) tmem_alloc(smem_u32(tm_slot), TMEM_COLS);
     if (tid == 0) {
@@ -636,6 +641,7 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
         mbar_init(bbar, 1);
         for (int i = 0; i < MAX_STG; i++) used[i] = 0;
         *stop = 0;
+        if (!finite) atomicExch(a.err, NOT_FINITE);
         /* the B images, behind the other set-up; the MMA warp waits for them */
         fence_proxy_async();
         expect_tx(bbar, 2u * L.blo);
