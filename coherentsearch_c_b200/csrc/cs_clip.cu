@@ -148,6 +148,12 @@ __global__ void __launch_bounds__(NT) zdm_cols_kernel(const uint8_t *raw, int L,
     for (int c = threadIdx.x; c < nchan; c += NT) atomicAdd(cols + b * nchan + c, csum[c]);
 }
 
+/* stats_kernel's dynamic shared memory: reciprocals, samples, good samples */
+static size_t stats_smem(int L)
+{
+    return (size_t)(L + 2) * sizeof(double) + 2 * (size_t)L * sizeof(int);
+}
+
 struct BlockStats {
     int ngood;
     float lo, hi;            /* good samples lie strictly between */
@@ -503,8 +509,7 @@ static int clip_run(const uint8_t *d_raw, long long nspec, int nchan, int L, flo
     if (cudaSetDevice(device) != cudaSuccess) return -1;
     cudaStream_t st = (cudaStream_t)stream;
     const long long n = nblocks * L;
-    /* statistics kernel: reciprocals, samples, good samples */
-    const size_t smem = (size_t)(L + 2) * sizeof(double) + 2 * (size_t)L * sizeof(int);
+    const size_t smem = ck::stats_smem(L);
     int nbits = 1;                           /* of a zero-DM sum */
     while (nbits < 31 && ((long long)nchan * 255) >> nbits) nbits++;
     size_t off[5];
@@ -523,9 +528,13 @@ static int clip_run(const uint8_t *d_raw, long long nspec, int nchan, int L, flo
     float *ravg = (float *)(base + off[2]), *trig = (float *)(base + off[3]);
     unsigned long long *cnt = (unsigned long long *)(base + off[4]), hcnt = 0;
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), st);
-    if (e == cudaSuccess && smem > 48 * 1024)
+    /* the limit of 48 KB is for this and the kernel's own arrays together.  It is
+     * raised to the longest block's need, never to this call's: a thread with other
+     * blocks may launch between the two calls */
+    if (e == cudaSuccess && smem > 32 * 1024)
         e = cudaFuncSetAttribute((const void *)ck::stats_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ck::stats_smem(ck::MAX_L));
     if (e == cudaSuccess) {
         const int vec16 = (nchan % 16 == 0) && (((uintptr_t)d_raw & 15) == 0);
         /* one pass for both sums where the levels are wanted and a warp's
