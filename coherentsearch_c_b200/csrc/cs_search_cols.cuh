@@ -897,7 +897,9 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
             }
         }
         if (!ok) fail();
-        /* never leave with copies in flight: the last use of each stage landed */
+        /* never leave with copies in flight: the last table and the last use of each
+         * stage landed.  Not full_wait, which ends when any role has given up */
+        if (loads && !mbar_wait(tbar, (loads - 1) & 1)) fail();
         for (int k = n > g.nstg ? n - g.nstg : 0; k < n; k++)
             if (!mbar_wait(wfull + 8 * (k % g.nstg), (k / g.nstg) & 1)) fail();
     } else if (warp == WARP_ROW) {
