@@ -602,10 +602,10 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
     const uint32_t wfull = bar, wempty = wfull + 8 * MAX_STG, afull = wempty + 8 * MAX_STG,
                    aempty = afull + 8 * NA, dfull = aempty + 8 * NA, dempty = dfull + 8 * MAX_ACC,
                    rfull = dempty + 8 * MAX_ACC, rempty = rfull + 8 * NROW, tbar = rempty + 8 * NROW,
-                   bbar = tbar + 8;
+                   bbar = tbar + 8, drain = bbar + 8;
     volatile int *stop = reinterpret_cast<volatile int *>(smem + L.bar + 496);
     uint32_t *tm_slot = reinterpret_cast<uint32_t *>(smem + L.bar + 500);
-    static_assert(8 * (2 * MAX_STG + 2 * NA + 2 * MAX_ACC + 2 * NROW + 2) <= 448, "barriers");
+    static_assert(8 * (2 * MAX_STG + 2 * NA + 2 * MAX_ACC + 2 * NROW + 3) <= 448, "barriers");
     /* uses of each window stage that its reader has begun with */
     volatile int *used = reinterpret_cast<volatile int *>(smem + L.bar + 448);
     static_assert(NACC >= 3 && NACC <= MAX_ACC, "the epilogue holds two accumulators");
@@ -639,6 +639,7 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
         }
         mbar_init(tbar, 1);
         mbar_init(bbar, 1);
+        mbar_init(drain, 1);
         for (int i = 0; i < MAX_STG; i++) used[i] = 0;
         *stop = 0;
         if (!finite) atomicExch(a.err, NOT_FINITE);
@@ -961,7 +962,6 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
                                    ((uint32_t)(CS_TILE_M >> 4) << 24);
             const uint32_t lbo_b = NPAD * 16;
             const uint32_t b_hi = sbase, b_lo = sbase + L.blo;
-            int last = -1;
             bool ok = full_wait(bbar, 0, 0);
             for (int it = 0; it < nt && ok; it++) {
                 const int s = it % NACC;
@@ -990,7 +990,6 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
                     wsk::mma_f16_ts(d, a_hi + 8 * k,
                                     umma_desc(b_hi + (uint32_t)k * 2 * lbo_b, lbo_b, 128), idesc, k > 0);
                     mma_commit(aempty + 8 * as);
-                    last = ks;
                 }
                 if (!ok) break;
                 for (int k = 0; k < NKS; k++)
@@ -1001,13 +1000,13 @@ __global__ void __launch_bounds__(Roles<C>::NTHREADS, 1) search_cols(const __gri
                                     umma_desc(b_lo + (uint32_t)k * 2 * lbo_b, lbo_b, 128), idesc, 1);
                 mma_commit(dfull + 8 * s);
             }
-            if (!ok) {
-                fail();
-                mbar_wait(bbar, 0);
-                /* never free tensor memory under work in flight (the tiles that went
-                 * through are waited for by the epilogue) */
-                if (last >= 0) mbar_wait(aempty + 8 * (last % NA), (last / NA) & 1);
-            }
+            if (!ok) fail();
+            /* never leave with the B images on their way, nor free tensor memory
+             * under copies and MMAs in flight, whichever role gave up */
+            bool landed = mbar_wait(bbar, 0);
+            mma_commit(drain);
+            landed = mbar_wait(drain, 0) && landed;
+            if (!landed) fail();
         }
     }
     __syncthreads();

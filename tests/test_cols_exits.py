@@ -25,3 +25,14 @@ def test_box_warps_wait_for_their_copies():
     for bar in issued:
         assert re.search(r"mbar_wait\(%s\b" % names.get(bar, bar), leave), bar
     assert "full_wait(" not in leave                # that one ends when any role gives up
+
+
+def test_mma_warp_waits_for_its_mmas():
+    """After the tile loop, on every way out of it: a commit behind all that was
+    issued, and a wait for it; the operand images are waited for too."""
+    text = role("--- MMAs ---", "tmem_dealloc")
+    leave = text[text.index("never leave with"):]
+    assert re.search(r"mma_commit\(drain\);\s*landed = mbar_wait\(drain, 0\)", leave)
+    assert "mbar_wait(bbar, 0)" in leave
+    before = text[:text.index("never leave with")]
+    assert before.rstrip().endswith("/*") and "if (!ok) {" not in before    # not only where it failed
