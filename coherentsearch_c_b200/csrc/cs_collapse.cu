@@ -35,7 +35,8 @@
  * candidates there that come before it in (r, chunk, slot, j) order (a
  * binary search): the stable r order of the (chunk, slot, j) base order.
  * The
- * metrics are FP32 values, so the metric sort uses 32-bit float keys.  The greedy
+ * metrics are FP32 values, so the metric sort uses 32-bit float keys (in shared
+ * memory up to CAP candidates, a device radix sort past that).  The greedy
  * pass runs in one CTA: for each kept candidate, in metric order, the threads mark every later
  * candidate it is related to; a candidate is kept when no earlier kept one
  * marked it, as in the host loop.  The FP64 expressions are the host's.
@@ -208,8 +209,14 @@ static __device__ __forceinline__ bool related_at(double r1, double r2, int mm, 
 
 static __device__ bool related(double r1, double r2, int numharm, double tol)
 {
-    for (int mm = 1; mm <= numharm; mm++)
-        if (related_at(r1, r2, mm, numharm, tol)) return true;
+    const double lo = r1 < r2 ? r1 : r2;
+    const double hi = r1 < r2 ? r2 : r1;
+    if (!(lo > 0.0)) return false;
+    for (int mm = 1; mm <= numharm; mm++) {
+        const int nn = (int)rint((double)mm * hi / lo);
+        if (nn < 1 || nn > numharm) continue;
+        if (fabs((double)mm * hi - (double)nn * lo) <= tol * (double)mm) return true;
+    }
     return false;
 }
 
@@ -492,63 +499,98 @@ struct FinishSmem {
 };
 
 /* The last steps for a list in global memory, which the runs' bests give first
- * when there are any.  Lists past CAP are ranked by counting and walked in global
- * memory (the walk, not the ranking, is what they cost).  The first CAP of the
- * result also go to pinned memory, with the number: no copy, and one wait less. */
+ * when there are any.  `keep` says which candidates stay; null: found here for up to
+ * CAP of them, and a longer list is left for order_and_walk, with its length in
+ * nout[1].  The first CAP of the result also go to pinned memory, with the number: no
+ * copy, and one wait less. */
 __global__ void __launch_bounds__(FT) finish_kernel(unsigned *list, const unsigned long long *best,
                                                     const unsigned *bidx, const unsigned *mp,
                                                     int harm_remove, int numharm, double tol,
                                                     const double *r, const double *freq,
                                                     const double *metric, const int *nharm,
-                                                    unsigned *mpos, unsigned char *removed,
-                                                    unsigned char *keep, Candidate *out,
+                                                    const unsigned char *keep, Candidate *out,
                                                     Candidate *pinned, unsigned *nout)
 {
     extern __shared__ __align__(16) unsigned char fsm[];
     FinishSmem &sm = *reinterpret_cast<FinishSmem *>(fsm);
     const unsigned m = *mp;
-    const bool small = m <= CAP;
     if (best) {
         for (unsigned p = threadIdx.x; p < m; p += FT) list[p] = bidx[(unsigned)best[p]];
         __syncthreads();
     }
-    if (harm_remove && small) {
+    if (harm_remove && !keep) {
+        if (m > CAP) {
+            if (threadIdx.x == 0) {
+                nout[0] = 0;
+                nout[1] = m;
+            }
+            return;
+        }
         harmonics_keep(sm.f, sm.t.sort, m, numharm, tol, [&](unsigned p, float &mt, double &rr) {
             const unsigned c = list[p];
             mt = (float)metric[c];              /* FP32 values: exact */
             rr = r[c];
         });
-    } else if (harm_remove) {
-        for (unsigned p = threadIdx.x; p < m; p += FT) {
-            const float x = (float)metric[list[p]];
-            unsigned rank = 0;
-            for (unsigned i = 0; i < m; i++) {
-                const float y = (float)metric[list[i]];
-                rank += y > x || (y == x && i < p) ? 1u : 0u;
-            }
-            mpos[rank] = p;
-            removed[rank] = 0;
-        }
-        __syncthreads();
-        for (unsigned i = 0; i < m; i++) {
-            if (removed[i]) continue;           /* the same value in every thread */
-            const double ri = r[list[mpos[i]]];
-            for (unsigned j = i + 1 + threadIdx.x; j < m; j += FT)
-                if (!removed[j] && related(r[list[mpos[j]]], ri, numharm, tol)) removed[j] = 1;
-            __syncthreads();
-        }
-        for (unsigned q = threadIdx.x; q < m; q += FT) keep[mpos[q]] = !removed[q];
-        __syncthreads();
     }
     const unsigned n = emit_kept(
-        sm.f, m, [&](unsigned i) { return !harm_remove || (small ? sm.f.keep[i] : keep[i]); },
+        sm.f, m, [&](unsigned i) { return !harm_remove || (keep ? keep[i] : sm.f.keep[i]); },
         [&](unsigned i, unsigned o) {
             const unsigned c = list[i];
             const Candidate x = make_cand(r[c], freq[c], metric[c], nharm[c]);
             out[o] = x;
             if (o < CAP) pinned[o] = x;
         });
-    if (threadIdx.x == 0) *nout = n;
+    if (threadIdx.x == 0) {
+        nout[0] = n;
+        nout[1] = 0;
+    }
+}
+
+/* ---- remove_harmonics of more than CAP candidates ---- */
+/* metric keys of the list, for the stable descending sort */
+__global__ void metric_keys_kernel(const unsigned *list, const double *metric, unsigned n,
+                                   const unsigned *m, float *key, unsigned *pos)
+{
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    key[i] = i < *m ? (float)metric[list[i]] : -INFINITY;     /* FP32 values: exact */
+    pos[i] = i;
+}
+
+/* The greedy walk over the metric order (one CTA), serial in the list: up to
+ * WALK_SMEM candidates' r and marks are in shared memory, so that a step costs a
+ * shared read and not two dependent global ones. */
+constexpr unsigned WALK_SMEM = 8192;
+constexpr size_t WALK_BYTES = WALK_SMEM * (sizeof(double) + 1);
+__global__ void __launch_bounds__(FT) walk_kernel(const unsigned *list, const unsigned *pos,
+                                                  const double *r, const unsigned *mp, int numharm,
+                                                  double tol, unsigned char *removed,
+                                                  unsigned char *keep)
+{
+    extern __shared__ double wsm[];
+    const unsigned m = *mp;
+    auto walk = [&](unsigned char *rm, auto at) {
+        for (unsigned i = 0; i < m; i++) {
+            if (rm[i]) continue;                /* the same value in every thread */
+            const double ri = at(i);
+            for (unsigned j = i + 1 + threadIdx.x; j < m; j += FT)
+                if (!rm[j] && related(at(j), ri, numharm, tol)) rm[j] = 1;
+            __syncthreads();
+        }
+        for (unsigned q = threadIdx.x; q < m; q += FT) keep[pos[q]] = !rm[q];
+    };
+    unsigned char *rs = reinterpret_cast<unsigned char *>(wsm + WALK_SMEM);
+    for (unsigned j = threadIdx.x; j < m; j += FT) {
+        if (m <= WALK_SMEM) {
+            wsm[j] = r[list[pos[j]]];
+            rs[j] = 0;
+        } else {
+            removed[j] = 0;
+        }
+    }
+    __syncthreads();
+    if (m <= WALK_SMEM) walk(rs, [&](unsigned i) { return wsm[i]; });
+    else walk(removed, [&](unsigned i) { return r[list[pos[i]]]; });
 }
 
 /* ---- the whole collapse of up to CAP records in one CTA ----
@@ -950,6 +992,9 @@ static cudaError_t finish_prepare()
     e = cudaFuncSetAttribute((const void *)cl::finish_kernel,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(cl::FinishSmem));
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void *)cl::walk_kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::WALK_BYTES);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void *)cl::collapse_small,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(cl::SmallSmem));
@@ -967,12 +1012,14 @@ struct CsCollapse {
     double *r, *freq, *metric;
     int *nharm;
     unsigned *flag, *runid, *list;
-    unsigned *mpos;
+    float *mkey[2];
+    unsigned *mpos[2];
     unsigned char *removed, *keep;
     Candidate *out;
     unsigned *counters;             /* device: valid, runs; then per-slot counts and
                                        starts (CS_MAX_SLOT each) */
-    unsigned *h_counters;           /* pinned: the length of the list */
+    unsigned *h_counters;           /* pinned: the length of the list; of one that
+                                       order_and_walk has yet to do, or 0 */
     void *bins;                     /* Bins, for the longest list so far */
     size_t bins_bytes;
     Candidate *h_out;               /* pinned */
@@ -980,6 +1027,9 @@ struct CsCollapse {
     void *temp;
     size_t temp_bytes;
     unsigned pending_n;             /* records of the enqueued collapse */
+    unsigned *pending_list;         /* its list, and the harmonics' settings */
+    int numharm, device;
+    double harm_tol;
     /* collapse_small's list and status (pinned), and whether it is queued */
     Candidate *s_out;
     unsigned *s_status;
@@ -989,11 +1039,9 @@ struct CsCollapse {
 static void collapse_release_buffers(CsCollapse *w)
 {
     for (int b = 0; b < 2; b++) {
-        cudaFree(w->key[b]); cudaFree(w->idx[b]);
-        w->key[b] = nullptr; w->idx[b] = nullptr;
+        cudaFree(w->key[b]); cudaFree(w->idx[b]); cudaFree(w->mkey[b]); cudaFree(w->mpos[b]);
+        w->key[b] = nullptr; w->idx[b] = nullptr; w->mkey[b] = nullptr; w->mpos[b] = nullptr;
     }
-    cudaFree(w->mpos);
-    w->mpos = nullptr;
     cudaFree(w->bkey); cudaFree(w->slot_of); cudaFree(w->merged);
     w->bkey = nullptr; w->slot_of = nullptr; w->merged = nullptr;
     cudaFree(w->r); cudaFree(w->freq); cudaFree(w->metric); cudaFree(w->nharm);
@@ -1019,8 +1067,9 @@ static cudaError_t collapse_reserve(CsCollapse *w, size_t n)
     for (int b = 0; b < 2; b++) {
         AL(w->key[b], c * sizeof(uint64_t));
         AL(w->idx[b], c * sizeof(unsigned));
+        AL(w->mkey[b], c * sizeof(float));
+        AL(w->mpos[b], c * sizeof(unsigned));
     }
-    AL(w->mpos, c * sizeof(unsigned));
     AL(w->bkey, c * sizeof(uint64_t));
     AL(w->slot_of, c * sizeof(int));
     AL(w->merged, c * sizeof(unsigned));
@@ -1038,13 +1087,16 @@ static cudaError_t collapse_reserve(CsCollapse *w, size_t n)
 #undef AL
     if (e != cudaSuccess) return e;
     /* the largest CUB scratch any step needs at this capacity */
-    size_t t1 = 0, t3 = 0;
+    size_t t1 = 0, t2 = 0, t3 = 0;
     cub::DoubleBuffer<uint64_t> kb(w->key[0], w->key[1]);
     cub::DoubleBuffer<unsigned> ib(w->idx[0], w->idx[1]);
+    cub::DoubleBuffer<float> mb(w->mkey[0], w->mkey[1]);
+    cub::DoubleBuffer<unsigned> pb(w->mpos[0], w->mpos[1]);
     e = cub::DeviceRadixSort::SortPairs(nullptr, t1, kb, ib, (int)c);
+    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairsDescending(nullptr, t2, mb, pb, (int)c);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, t3, w->flag, w->runid, (int)c);
     if (e != cudaSuccess) return e;
-    w->temp_bytes = std::max(t1, t3);
+    w->temp_bytes = std::max(t1, std::max(t2, t3));
     e = cudaMalloc(&w->temp, w->temp_bytes);
     if (e == cudaSuccess) w->cap = c;
     return e;
@@ -1200,6 +1252,29 @@ static bool bins_for(CsCollapse *w, unsigned n, long long nchunks, const cl::Slo
     return cudaMemsetAsync(w->bins, 0xFF, ones, st) == cudaSuccess;
 }
 
+/* keep[] of a list of up to n candidates, any length: the radix sort by metric,
+ * then the walk.  (Ranked by counting in one CTA, a list of
+ * 53 k records took 243 ms in all and one of 200 k 3.0 s; so 41 and 179 ms.) */
+static cudaError_t order_and_walk(CsCollapse *w, const unsigned *list, unsigned n, int numharm,
+                                  double tol, cudaStream_t st)
+{
+    const unsigned *m = w->counters + 1;
+    cub::DoubleBuffer<float> mb(w->mkey[0], w->mkey[1]);
+    cub::DoubleBuffer<unsigned> pb(w->mpos[0], w->mpos[1]);
+    size_t tb = w->temp_bytes;
+    cl::metric_keys_kernel<<<(n + cl::NT - 1) / cl::NT, cl::NT, 0, st>>>(list, w->metric, n, m,
+                                                                        w->mkey[0], w->mpos[0]);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cub::DeviceRadixSort::SortPairsDescending(w->temp, tb, mb, pb, (int)n, 0, 32, st);
+    if (e == cudaSuccess) {
+        cl::walk_kernel<<<1, cl::FT, cl::WALK_BYTES, st>>>(list, pb.Current(), w->r, m, numharm, tol,
+                                                           w->removed, w->keep);
+        e = cudaGetLastError();
+    }
+    return e;
+}
+
 int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsChunk *chunks,
                         long long nchunks, const int *slot_k, const int *slot_Hk, int nslot,
                         int nprof, double r_lo, double lodr, double N, double T,
@@ -1285,11 +1360,19 @@ int cs_collapse_enqueue(CsCollapse *w, const CsRec *recs, unsigned n, const CsCh
             list = w->merged;
         }
     }
+    w->pending_list = list;
+    w->numharm = numharm;
+    w->harm_tol = harm_tol;
+    if (e == cudaSuccess) e = cudaGetDevice(&w->device);
+    /* with every record in the list it is too long for finish_kernel; after
+     * remove_duplicates it seldom is, and cs_collapse_finish sees to that */
+    const bool all = harm_remove && !remove && n > cl::CAP;
+    if (e == cudaSuccess && all) e = order_and_walk(w, list, n, numharm, harm_tol, st);
     if (e == cudaSuccess) {
         cl::finish_kernel<<<1, cl::FT, sizeof(cl::FinishSmem), st>>>(
             list, binned ? bn.best : nullptr, binned ? bn.idx : nullptr, m, harm_remove, numharm,
-            harm_tol, w->r, w->freq, w->metric, w->nharm, w->mpos, w->removed, w->keep, w->out,
-            w->s_out, w->h_counters);
+            harm_tol, w->r, w->freq, w->metric, w->nharm, all ? w->keep : nullptr, w->out, w->s_out,
+            w->h_counters);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -1317,6 +1400,22 @@ int cs_collapse_finish(CsCollapse *w, cudaStream_t st, CandidateList *out)
             out->cap = nout;
         }
         return 0;
+    }
+    if (w->h_counters[1]) {
+        int here = w->device;                   /* the waiting thread may be on another */
+        e = cudaGetDevice(&here);
+        if (e == cudaSuccess) e = cudaSetDevice(w->device);
+        if (e == cudaSuccess)
+            e = order_and_walk(w, w->pending_list, w->h_counters[1], w->numharm, w->harm_tol, st);
+        if (e == cudaSuccess) {
+            cl::finish_kernel<<<1, cl::FT, sizeof(cl::FinishSmem), st>>>(
+                w->pending_list, nullptr, nullptr, w->counters + 1, 1, w->numharm, w->harm_tol, w->r,
+                w->freq, w->metric, w->nharm, w->keep, w->out, w->s_out, w->h_counters);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (here != w->device) cudaSetDevice(here);
+        if (e != cudaSuccess) goto fail;
     }
     {
         const unsigned nout = w->h_counters[0];
