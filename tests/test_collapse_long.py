@@ -82,3 +82,14 @@ def test_ordering_does_not_grow_with_the_square(gpu_ready, remove):
         assert 0 < n < want // 8
         took.append(t)
     assert took[1] < 22.0 * took[0]                 # between linear, 8, and the square, 64
+
+
+@pytest.mark.gpu
+def test_one_launch_is_not_the_slower_one(gpu_ready):
+    """Noise, some hundred candidates kept: a list just short enough for one launch
+    against one just past it, whose walk is the plain one."""
+    N, wants = 400000, (4090, 4110)
+    amps = _spectrum(N, 6)
+    short, long = (_time(N, amps, thr, Options(threshold=thr), False, 1.0)[0]
+                   for thr in _thresholds(N, amps, wants))
+    assert short < 1.05 * long
