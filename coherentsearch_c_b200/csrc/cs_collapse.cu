@@ -306,10 +306,11 @@ static __device__ void harmonics_keep(FinishShared &f, MetricSort::TempStorage &
      * step being one FP64 division deep and not numharm of them (40 candidates, 4
      * kept: 20 k cycles -> 8 k).  (What 53 k records of noise
      * leave after remove_duplicates: 3.14 ms with pairs all the way, 2.33 so; 4 k
-     * trials of one pulsar 344 us and 305.) */
+     * trials of one pulsar 344 us and 305.)  Harmonics past 2^31 / FT never pair:
+     * the number of pairs stays in 32 bits. */
     const unsigned nh = numharm > 0 ? (unsigned)numharm : 0u;
     unsigned i = next(0);
-    for (; i < m && m - i - 1 > FT / 2; i = next(i + 1)) {
+    for (; i < m && (m - i - 1 > FT / 2 || nh > (1u << 31) / FT); i = next(i + 1)) {
         const double ri = f.rs[i];
         for (unsigned j = i + 1 + tid; j < m; j += FT)
             if (!f.rm[j] && related(f.rs[j], ri, numharm, tol)) f.rm[j] = 1;

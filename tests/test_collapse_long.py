@@ -93,3 +93,21 @@ def test_one_launch_is_not_the_slower_one(gpu_ready):
     short, long = (_time(N, amps, thr, Options(threshold=thr), False, 1.0)[0]
                    for thr in _thresholds(N, amps, wants))
     assert short < 1.05 * long
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("numharm", [1 << 19, 1 << 21, (1 << 21) + 1, 1 << 24])
+@pytest.mark.parametrize("want", [300, 1500, 4500])
+def test_many_harmonics(gpu_ready, want, numharm):
+    """Numbers of (candidate, harmonic) pairs around 2^31 and past 2^32."""
+    N = 60000
+    amps = _spectrum(N, want)
+    thr, = _thresholds(N, amps, [want])
+    ses = Session(N, 64e-6, Options(threshold=thr, blocksize=5000, numharm=numharm, remove=False))
+    host = ses.collapse(ses.run_raw(amps))
+    ses.enqueue(None)
+    got, _, rc = ses.collect_collapsed()
+    ses.close()
+    assert rc == 0 and 0 < host.size < want // 4
+    for f in ("freq", "metric", "r", "nharm"):
+        np.testing.assert_array_equal(got[f], host[f])
