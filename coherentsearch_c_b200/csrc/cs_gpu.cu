@@ -1273,10 +1273,24 @@ static bool cols_geometry(const CsTables &t, long long total, long long namps, i
     return g.nstg >= MIN_STG;
 }
 
+/* Bytes of a search_cols session's own buffer, in this order: tensor maps, tables
+ * of npb phase blocks, padded copy of the spectrum (shift: the bins between columns
+ * of the last harmonic). */
+static size_t cols_bytes(int npb, int tab_bytes, long long namps, long long shift,
+                         size_t *tab_off = nullptr, size_t *pad_off = nullptr)
+{
+    const size_t tab = sizeof(CUtensorMap) * wsk::MAX_NH;
+    const size_t pad = tab + (size_t)npb * tab_bytes;                  /* multiples of 128 */
+    if (tab_off) *tab_off = tab;
+    if (pad_off) *pad_off = pad;
+    return pad + (cols::FRONT + (size_t)namps + 7 * (size_t)shift + 64) * sizeof(float2);
+}
+
 /* Tables, padded copy and tensor maps of the register-block kernel; false
  * (with the session left on search_ws or the generic kernel) when the
- * geometry does not fit or any step is refused. */
-static bool cols_load(GpuSession *S, const CsTables &t, long long total)
+ * geometry does not fit, the buffer would grow by more than `room` bytes or any
+ * step is refused. */
+static bool cols_load(GpuSession *S, const CsTables &t, long long total, size_t room)
 {
     using namespace cols;
     const int nh = ladder_config(t, total);
@@ -1288,10 +1302,10 @@ static bool cols_load(GpuSession *S, const CsTables &t, long long total)
     S->cols_smem = layout(g, t.npad, t.kpad).total;
     const size_t back = 7 * (size_t)g.shift[nh - 1] + 64;
     const size_t nbins = FRONT + (size_t)S->namps + back;
-    const size_t tab_off = sizeof(CUtensorMap) * wsk::MAX_NH;
-    const size_t pad_off = tab_off + (size_t)g.npb * g.tab_bytes;      /* multiples of 128 */
-    if (dev_reserve((void **)&S->d_cols, &S->c_cols, pad_off + nbins * sizeof(float2)) != cudaSuccess)
-        return false;
+    size_t tab_off, pad_off;
+    const size_t need = cols_bytes(g.npb, g.tab_bytes, S->namps, g.shift[nh - 1], &tab_off, &pad_off);
+    if (need > S->c_cols && need - S->c_cols > room) return false;
+    if (dev_reserve((void **)&S->d_cols, &S->c_cols, need) != cudaSuccess) return false;
     S->d_pad = (float2 *)(S->d_cols + pad_off);
     if (!S->h_cmaps)
         S->h_cmaps = (CUtensorMap *)aligned_alloc(64, sizeof(CUtensorMap) * wsk::MAX_NH);
@@ -1408,7 +1422,8 @@ static cudaError_t set_smem_cap(const void *fn, int max_optin)
  * (callers release it). */
 static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
                         const DirectPlanSet *dplans, const long long *cstarts, long long total,
-                        int Nprof, long long nchunks, double r_lo, double lodr)
+                        int Nprof, long long nchunks, double r_lo, double lodr,
+                        size_t cols_room = SIZE_MAX)
 {
     char err[512] = {0};
     std::vector<uint16_t> bhi, blo;
@@ -1567,7 +1582,7 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
     S->use_tma = S->use_tci ? 0 : tma_config(t, total, S->namps, S->use_ws);
     if (S->use_tma && (tma_smem(S->use_tma) > S->max_smem || !tma_load(S, t, total)))
         S->use_tma = 0;
-    if (!S->use_tci && !S->use_tma) (void)cols_load(S, t, total);
+    if (!S->use_tci && !S->use_tma) (void)cols_load(S, t, total, cols_room);
     (void)cudaGetLastError();
     {
         /* Start with room for 1 in 16 trials per slot; grown on overflow. */
@@ -2781,6 +2796,7 @@ struct BatchReq {
     bool rekeyed;                    /* the slot's tables were rebuilt for it */
     int only_slot = -1;              /* >= 0: only this slot takes it */
     bool load_only = false;          /* build tables and buffers, no search */
+    size_t cols_room = SIZE_MAX;     /* device bytes left for search_cols' buffer */
     std::chrono::steady_clock::time_point t_submit, t_start, t_admit, t_loaded, t_end;
 };
 
@@ -2835,6 +2851,22 @@ static size_t batch_footprint(const BatchReq *r, long long total, int Nprof)
     return (size_t)r->ft.namps * sizeof(float2) + (size_t)recs * sizeof(CsRec) +
            (size_t)(total / CS_TILE_M + nchunks + 1) * 3 * sizeof(int) +
            (size_t)nchunks * sizeof(CsChunk) + ((size_t)4 << 20);
+}
+
+/* The most that search_cols adds to it where it takes the request: it runs with
+ * what the budget leaves over, and the search does without where that is less. */
+static size_t batch_cols(const BatchReq *r, double lodr)
+{
+    int p = 0, q = 0;
+    const int nh = r->p.nharms;
+    if ((nh != 60 && nh != 32 && nh != 16) || r->p.m != wsk::M || r->p.precision != 0 ||
+        !trial_grid_rational(lodr, &p, &q))
+        return 0;
+    long long D = 2LL * q;
+    while (D % cols::TI) D += 2LL * q;
+    if (D > 4096) return 0;
+    const int tab = (nh * cols::TI * (20 * 4 + 8) + 512 + 127) / 128 * 128;
+    return cols_bytes((int)(D / cols::TI), tab, r->ft.namps, (long long)nh * p * (D / q));
 }
 
 /* Admit slot k for a request needing `need` bytes: wait (lock held by the
@@ -2913,7 +2945,7 @@ static void batch_run_one(CsBatch *B, int k, BatchReq *r)
         if (direct_plans_build(&plans, &r->p, r_lo) != 0) return;
         const int rc = chunk_starts(&plans, &r->ft, &r->p, total, Nprof, &cstarts, &nchunks);
         const int lrc = rc == 0 ? session_load(S, &r->ft, &r->p, &plans, cstarts, total, Nprof,
-                                               nchunks, r_lo, lodr)
+                                               nchunks, r_lo, lodr, r->cols_room)
                                 : -1;
         free(cstarts);
         direct_plans_free(&plans);
@@ -2980,6 +3012,12 @@ static void batch_worker(CsBatch *B, int k)
             B->slots[k].busy = true;
             /* reserve the room while the slot grows into it */
             B->slots[k].bytes = std::max(B->slots[k].bytes, need);
+            if (B->budget) {
+                size_t held = 0;
+                for (const BatchSlot &o : B->slots) held += o.bytes;
+                r->cols_room = std::min(B->budget - held, need ? batch_cols(r, lodr) : 0);
+                B->slots[k].bytes += r->cols_room;
+            }
             lk.unlock();
             r->t_admit = r->t_loaded = std::chrono::steady_clock::now();
             batch_run_one(B, k, r);
