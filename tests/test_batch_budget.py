@@ -38,14 +38,20 @@ def test_slots_hold_what_was_admitted(gpu_ready, slots, spare):
     nt.gpu_lib().cs_b200_session_park_drain()
     budget, seen, stop = int(spare * _needs(N)), [], threading.Event()
     with Batch(nslots=slots, mem_budget=budget) as b:
-        watch = threading.Thread(target=lambda: [seen.append(b.device_bytes())
-                                                 for _ in iter(stop.is_set, True)])
+        def look():
+            while not stop.is_set():
+                seen.append(b.device_bytes())
+                stop.wait(2e-4)
+
+        watch = threading.Thread(target=look, daemon=True)
         watch.start()
-        ids = [b.submit(data[i % 3], N, DT, OPTS) for i in range(9)]
-        got = [b.wait(i)[0] for i in ids]
+        try:
+            ids = [b.submit(data[i % 3], N, DT, OPTS) for i in range(9)]
+            got = [b.wait(i)[0] for i in ids]
+        finally:                                    # also where a request failed
+            stop.set()
+            watch.join()
         seen.append(b.device_bytes())
-        stop.set()
-        watch.join()
     for i, g in enumerate(got):
         for f in ("r", "metric", "nharm"):
             np.testing.assert_array_equal(g[f], want[i % 3][f])
