@@ -865,13 +865,28 @@ static int grow_records64(GpuSession *S, unsigned cap)
     return 0;
 }
 
+/* Give search_cols' buffer back (the session searches without it); false: there was none. */
+static bool cols_drop(GpuSession *S)
+{
+    if (!S->d_cols) return false;
+    cudaFree(S->d_cols);
+    S->d_cols = NULL;
+    S->c_cols = 0;
+    S->use_cols = 0;
+    (void)cudaGetLastError();
+    return true;
+}
+
 static int grow_records(GpuSession *S, unsigned cap)
 {
     S->gen++;
     cudaFree(S->d_recs);
     S->d_recs = NULL;
     S->cap = 0;
-    if (cudaMalloc((void **)&S->d_recs, (size_t)cap * sizeof(CsRec)) != cudaSuccess) {
+    /* the records come before what only makes the search faster */
+    const size_t bytes = (size_t)cap * sizeof(CsRec);
+    if (cudaMalloc((void **)&S->d_recs, bytes) != cudaSuccess &&
+        !(cols_drop(S) && cudaMalloc((void **)&S->d_recs, bytes) == cudaSuccess)) {
         fprintf(stderr, "Error: cannot allocate %u candidate records on the GPU\n", cap);
         return -1;
     }
@@ -1530,8 +1545,14 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
         CK(dev_reserve((void **)&S->d_scales, &S->c_scales, nsc * sizeof(double)));
         CK(cudaMemcpyAsync(S->d_scales, t.invsw64, nsc * sizeof(double), cudaMemcpyHostToDevice,
                            S->st));
+        if (S->f64_wide && t.m == 16 &&
+            dev_reserve((void **)&S->d_wt64, &S->c_wt64, (size_t)t.nrows * t.m * sizeof(float)) !=
+                cudaSuccess) {
+            (void)cudaGetLastError();
+            S->f64_wide = 0;
+            S->f64_smem = f64k::smem_bytes(t.nh, x.ucols, x.prs, x.ps_total);
+        }
         if (S->f64_wide && t.m == 16) {
-            CK(dev_reserve((void **)&S->d_wt64, &S->c_wt64, (size_t)t.nrows * t.m * sizeof(float)));
             CK(cudaMemcpyAsync(S->d_wt64, t.Wt, (size_t)t.nrows * t.m * sizeof(float),
                                cudaMemcpyHostToDevice, S->st));
             x.wt = S->d_wt64;
@@ -1582,8 +1603,6 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
     S->use_tma = S->use_tci ? 0 : tma_config(t, total, S->namps, S->use_ws);
     if (S->use_tma && (tma_smem(S->use_tma) > S->max_smem || !tma_load(S, t, total)))
         S->use_tma = 0;
-    if (!S->use_tci && !S->use_tma) (void)cols_load(S, t, total, cols_room);
-    (void)cudaGetLastError();
     {
         /* Start with room for 1 in 16 trials per slot; grown on overflow. */
         long long want = (total * t.nslot) / 16 + 4096;
@@ -1591,6 +1610,9 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
         if (!S->d_recs || S->cap < (unsigned)want)
             if (grow_records(S, (unsigned)want) != 0) return -1;
     }
+    /* last of the buffers: a session that fits without it is made without it */
+    if (!S->use_tci && !S->use_tma) (void)cols_load(S, t, total, cols_room);
+    (void)cudaGetLastError();
     /* the cap is per kernel, not per session: sessions of other geometries may
      * launch concurrently (batch slots), so it is set to the device limit,
      * never lowered to this geometry's need */
