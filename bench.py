@@ -1159,7 +1159,7 @@ def sweep_lines(files, slots, nh_list, steps, warmup, ref_gpu, device=0):
         # launch over all their tiles (the kernel-side bound of the grouped form)
         for i in range(len(specs)):
             upload(i)
-        resident = [Session(sp.N, dt, opts, device=device) for sp in specs]
+        resident = [Session(sp.N, dt, opts, device=device, multi=True) for sp in specs]
         ptrs = [b.data_ptr() for b in dev_bufs]
         try:
             multi_search(resident, ptrs, stream=st)                # warm

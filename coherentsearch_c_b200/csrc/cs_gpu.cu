@@ -1715,11 +1715,10 @@ CS_EXPORT int cs_b200_session_park_drain(void)
     return (int)all.size();
 }
 
-CS_EXPORT GpuSession *cs_gpu_session_create(const FFTFile *ft, const SearchParams *p,
-                                            const DirectPlanSet *dplans,
-                                            const long long *cstarts, long long total,
-                                            int Nprof, long long nchunks, double r_lo,
-                                            double lodr, int device)
+static GpuSession *session_create(const FFTFile *ft, const SearchParams *p,
+                                  const DirectPlanSet *dplans, const long long *cstarts,
+                                  long long total, int Nprof, long long nchunks, double r_lo,
+                                  double lodr, int device, size_t cols_room)
 {
     GpuSession *S = park_take(device);
     if (S) {
@@ -1731,11 +1730,31 @@ CS_EXPORT GpuSession *cs_gpu_session_create(const FFTFile *ft, const SearchParam
         S = session_new(device);
     }
     if (!S) return NULL;
-    if (session_load(S, ft, p, dplans, cstarts, total, Nprof, nchunks, r_lo, lodr) != 0) {
+    if (session_load(S, ft, p, dplans, cstarts, total, Nprof, nchunks, r_lo, lodr, cols_room) != 0) {
         session_release(S);
         return NULL;
     }
     return S;
+}
+
+CS_EXPORT GpuSession *cs_gpu_session_create(const FFTFile *ft, const SearchParams *p,
+                                            const DirectPlanSet *dplans,
+                                            const long long *cstarts, long long total,
+                                            int Nprof, long long nchunks, double r_lo,
+                                            double lodr, int device)
+{
+    return session_create(ft, p, dplans, cstarts, total, Nprof, nchunks, r_lo, lodr, device,
+                          SIZE_MAX);
+}
+
+CS_EXPORT GpuSession *cs_b200_session_create_multi(const FFTFile *ft, const SearchParams *p,
+                                                   const DirectPlanSet *dplans,
+                                                   const long long *cstarts, long long total,
+                                                   int Nprof, long long nchunks, double r_lo,
+                                                   double lodr, int device)
+{
+    /* no room to grow: a parked session's buffer that is large enough is used */
+    return session_create(ft, p, dplans, cstarts, total, Nprof, nchunks, r_lo, lodr, device, 0);
 }
 
 CS_EXPORT int cs_gpu_session_matches(const GpuSession *S, const FFTFile *ft,

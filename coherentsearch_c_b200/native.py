@@ -129,6 +129,8 @@ def declare_gpu_api(lib: C.CDLL) -> C.CDLL:
                                           P(C.c_longlong), C.c_longlong, C.c_int, C.c_longlong,
                                           C.c_double, C.c_double, C.c_int]
     lib.cs_gpu_session_create.restype = C.c_void_p
+    lib.cs_b200_session_create_multi.argtypes = lib.cs_gpu_session_create.argtypes
+    lib.cs_b200_session_create_multi.restype = C.c_void_p
     lib.cs_gpu_session_matches.argtypes = [C.c_void_p, P(FFTFile), P(SearchParams), C.c_int,
                                            C.c_longlong, C.c_double, C.c_double, C.c_int]
     lib.cs_gpu_session_matches.restype = C.c_int

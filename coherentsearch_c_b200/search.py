@@ -120,9 +120,12 @@ def search_spectrum(amps, N: int, dt: float, opts: Options | None = None,
 
 
 class Session:
-    """Plans + one GPU session for spectra of a fixed geometry (N, dt, options)."""
+    """Plans + one GPU session for spectra of a fixed geometry (N, dt, options).
+    `multi`: for multi_enqueue, MultiGraph and the allocation-free search, without the
+    buffers that only searches of one spectrum use (cs_b200_session_create_multi)."""
 
-    def __init__(self, N: int, dt: float, opts: Options | None = None, device: int = 0):
+    def __init__(self, N: int, dt: float, opts: Options | None = None, device: int = 0,
+                 multi: bool = False):
         self.opts = opts or Options()
         self.N, self.dt, self.device = N, dt, device
         self.host = nt.host_lib()
@@ -148,11 +151,12 @@ class Session:
         self.cstarts = np.ctypeslib.as_array(cs, shape=(self.nchunks,)).copy()
         _libc_free(cs)
         self._cs = self.cstarts.ctypes.data_as(C.POINTER(C.c_longlong))
-        self.sess = self.gpu.cs_gpu_session_create(
+        create = self.gpu.cs_b200_session_create_multi if multi else self.gpu.cs_gpu_session_create
+        self.sess = create(
             C.byref(self.ft), C.byref(self.params), C.byref(self.plans), self._cs, self.total,
             self.opts.blocksize, self.nchunks, self.r_lo, self.lodr, device)
         if not self.sess:
-            raise RuntimeError("cs_gpu_session_create failed (see stderr)")
+            raise RuntimeError("session_create failed (see stderr)")
 
     def info(self) -> nt.CsB200Info:
         inf = nt.CsB200Info()

@@ -44,7 +44,7 @@ def search_list(spectra, dt: float, opts: Options, group: int, device: int = 0,
     for g0 in range(0, n, max(1, group)):
         idx = list(range(g0, min(n, g0 + group)))
         # host tables of this group while the previous group's kernel runs
-        sess = [Session(spectra[i][0], dt, opts, device=device) for i in idx]
+        sess = [Session(spectra[i][0], dt, opts, device=device, multi=True) for i in idx]
         ptrs = [upload(i) if upload else spectra[i][1] for i in idx]
         # queued behind the previous launch; its harvest then overlaps this one
         multi_enqueue(sess, ptrs, stream=stream)
@@ -61,7 +61,7 @@ def warm(max_n: int, dt: float, opts: Options, count: int, device: int = 0) -> N
     the groups of search_list reload them without growing a device buffer
     (a cudaFree waits for the whole device).  The park must hold `count`
     (CS_B200_SESSION_PARK); cs_b200_session_park_drain gives the memory back."""
-    sess = [Session(max_n, dt, opts, device=device) for _ in range(count)]
+    sess = [Session(max_n, dt, opts, device=device, multi=True) for _ in range(count)]
     for s in sess:
         s.close()
 

@@ -36,6 +36,15 @@ typedef struct {
 
 int cs_b200_session_info(const GpuSession *s, CsB200Info *info);
 
+/* cs_gpu_session_create for sessions that are searched by cs_b200_multi_enqueue,
+ * cs_b200_multi_graph_* or cs_b200_session_search_noalloc: without the tables and the
+ * second copy of the spectrum (8 bytes a bin) that only a search of one spectrum by
+ * itself uses.  Such a search works too, on the kernel those calls launch. */
+GpuSession *cs_b200_session_create_multi(const FFTFile *ft, const SearchParams *p,
+                                         const DirectPlanSet *dplans, const long long *cstarts,
+                                         long long total, int Nprof, long long nchunks,
+                                         double r_lo, double lodr, int device);
+
 /* One persistent launch over the tiles of several spectra (no counterpart
  * in the reference, which searches one file per call): sessions ss[0..n-1],
  * all FP32 and of one warp-specialised configuration (the same nharms and
