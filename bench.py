@@ -55,8 +55,11 @@ DFT_FLOP_PER_TRIAL = 28560.0      # 2*(2nh-1)*2nh at nh=60 (k | nh folds add non
 SIMT_OPS_PER_TRIAL = 6000.0       # interp 1920 FMA + 360 rotate + boxcar/fold ~3700
 
 
-KERNEL_NAMES = {0: "cs_search_kernel", 1: "search_cols_cfg60", 2: "search_f64",
-                3: "search_tma_cfg60", 4: "interp_tc + search_pre_cfg60"}
+def kernel_label(ses):
+    """The search kernel of a session, with its configuration where it has one."""
+    name = ses.kernel_name()
+    cfg = name in ("search_cols", "search_ws", "search_tma", "interp_tc + search_pre")
+    return f"{name}_cfg{ses.opts.nharms}" if cfg else name
 
 
 def cpu_model():
@@ -532,7 +535,7 @@ def run_b200(args):
     f_sm = (clocks.get("sm_mhz") or 1965.0) * 1e6
     simt_peak = 148 * 128 * f_sm
     simt_ach = total * SIMT_OPS_PER_TRIAL / (kms * 1e-3)
-    kname = KERNEL_NAMES.get(info.kernel, "unknown")
+    kname = kernel_label(ses)
     traffic = profiled_traffic(kname, total)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
@@ -800,7 +803,8 @@ def dedisp_measure(args, world, rank, local, pg):
         "roofline": {"bound": "hbm", "achieved": alg_bytes / (kern_ms * 1e-3) / 1e9,
                      "peak": hbm_peak, "unit": "GB/s",
                      "frac": alg_bytes / (kern_ms * 1e-3) / 1e9 / hbm_peak, "traffic": None,
-                     "kernel": ("dd_subband_clip + dd_dms_f32" if args.clipped
+                     "kernel": ("dd_subband_u8 + dd_dms_u16, and dd_subband_clip + dd_dms_f32 "
+                                "where a replaced spectrum reaches" if args.clipped
                                 else "dd_subband_u8 + dd_dms_u16"),
                      "subband_ms": statistics.mean(sb_ms), "dm_ms": statistics.mean(dm_ms),
                      "peak_kind": f"HBM copy, {peak_kind}",
@@ -963,7 +967,7 @@ def run_prep(args):
         "gpu_launches": (7 + 6 * t.ndm) * args.steps,
         "roofline": {"bound": "tensor", "achieved": dft_tflops, "peak": tc_peak,
                      "unit": "TFLOP/s", "frac": dft_tflops / tc_peak, "traffic": None,
-                     "kernel": "search_cols_cfg60", "kernel_ms_per_dm": kms / t.ndm,
+                     "kernel": kernel_label(ps.sessions[0]), "kernel_ms_per_dm": kms / t.ndm,
                      "peak_kind": f"bf16 dense, {peak_kind}",
                      "algorithmic": f"{DFT_FLOP_PER_TRIAL:.0f} DFT flop/trial x {total} trials "
                                     f"x {t.ndm} DMs"},
@@ -1536,7 +1540,7 @@ def run_series(args):
         "gpu_launches": 6 * args.steps,      # 3 spectrum, 2 search, 1 collapse (cuFFT not counted)
         "roofline": {"bound": "tensor", "achieved": dft, "peak": tc_peak, "unit": "TFLOP/s",
                      "frac": dft / tc_peak, "traffic": None,
-                     "kernel": KERNEL_NAMES.get(ses.info().kernel, "unknown"),
+                     "kernel": kernel_label(ses),
                      "kernel_ms": kms, "peak_kind": f"bf16 dense, {peak_kind}"},
         "candidates": int(out.size),
         "clocks": clk.summary(),

@@ -2130,6 +2130,16 @@ CS_EXPORT int cs_b200_session_info(const GpuSession *S, CsB200Info *info)
     return 0;
 }
 
+CS_EXPORT const char *cs_b200_session_kernel_name(const GpuSession *S)
+{
+    if (!S) return "";
+    if (S->prec64) return S->f64_wide ? "search_f64_wide" : "search_f64";
+    if (S->use_tci) return "interp_tc + search_pre";
+    if (S->use_tma) return "search_tma";
+    if (S->use_cols) return "search_cols";
+    return S->use_ws ? "search_ws" : "cs_search_kernel";
+}
+
 CS_EXPORT int cs_b200_session_enqueue_device(GpuSession *S, const float *d_amps,
                                              double threshold, void *stream)
 {

@@ -143,6 +143,8 @@ def declare_gpu_api(lib: C.CDLL) -> C.CDLL:
     lib.cs_gpu_search_region.restype = CandidateList
     lib.cs_b200_session_info.argtypes = [C.c_void_p, P(CsB200Info)]
     lib.cs_b200_session_info.restype = C.c_int
+    lib.cs_b200_session_kernel_name.argtypes = [C.c_void_p]
+    lib.cs_b200_session_kernel_name.restype = C.c_char_p
     lib.cs_b200_session_device_amps.argtypes = [C.c_void_p]
     lib.cs_b200_session_device_amps.restype = C.c_void_p
     lib.cs_b200_multi_enqueue.argtypes = [C.POINTER(C.c_void_p), C.c_int,

@@ -163,6 +163,10 @@ class Session:
         self.gpu.cs_b200_session_info(self.sess, C.byref(inf))
         return inf
 
+    def kernel_name(self) -> str:
+        """The kernel a search of one spectrum launches (cs_b200_session_kernel_name)."""
+        return self.gpu.cs_b200_session_kernel_name(self.sess).decode()
+
     def run_raw(self, amps, threshold: float | None = None) -> np.ndarray:
         """cs_gpu_session_run: uncollapsed candidates in the reference order."""
         a = _as_amps(amps)

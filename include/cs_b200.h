@@ -36,6 +36,12 @@ typedef struct {
 
 int cs_b200_session_info(const GpuSession *s, CsB200Info *info);
 
+/* The kernel that a search of one finite spectrum by this session launches:
+ * "search_cols", "search_ws" (where search_cols' geometry or memory does not fit),
+ * "search_tma", "interp_tc + search_pre", "cs_search_kernel", "search_f64_wide" or
+ * "search_f64" (a constant string). */
+const char *cs_b200_session_kernel_name(const GpuSession *s);
+
 /* cs_gpu_session_create for sessions that are searched by cs_b200_multi_enqueue,
  * cs_b200_multi_graph_* or cs_b200_session_search_noalloc: without the tables and the
  * second copy of the spectrum (8 bytes a bin) that only a search of one spectrum by
