@@ -1312,6 +1312,13 @@ static bool cols_load(GpuSession *S, const CsTables &t, long long total, size_t 
     if (!nh || S->prec64 || getenv("CS_B200_WS_KERNEL")) return false;
     Geo &g = S->cx.g;
     if (!cols_geometry(t, total, S->namps, S->max_smem, g)) return false;
+    /* Where the chip has less than a wave or two of tiles, search_cols' longer way in
+     * (a phase table and boxes before the first multiply) is not made up for.  Kernel,
+     * search_ws and search_cols: nharms 32 with 147 tiles 17.2 and 18.4 us, 157 22.6 and
+     * 18.4; nharms 16 with 269 16.5 and 18.3, 365 20.5 and 18.9; nharms 60 with 103
+     * 26.6 and 24.6. */
+    const int waves = nh == 16 ? 2 : nh == 32 ? 1 : 0;
+    if (S->use_ws && t.ntiles <= waves * S->nsm) return false;
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
     S->cols_smem = layout(g, t.npad, t.kpad).total;
