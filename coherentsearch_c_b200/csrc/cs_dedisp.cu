@@ -1435,14 +1435,39 @@ static ClipRoom dd_clip_room(const CsDedisp *D)
     return r;
 }
 
-/* The subband stage of one kind over the tiles up to sfill. */
-static cudaError_t dd_subbands(CsDedisp *D, dd::SubArgs sa, bool clip, long long sfill,
-                               cudaStream_t st)
+/* Subbands that a CTA of the subband stage takes. */
+static int dd_slab(const CsDedisp *D, bool clip)
 {
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, D->device);
     int slab = std::max(1, std::min(D->nsub, 256 / std::max(1, D->cps)));
     while (slab > 1 && sb_smem(D, slab, clip) > std::min(max_optin, 100 * 1024)) slab /= 2;
+    return slab;
+}
+
+/* Whether a clipped run is worth its second pair of stages: the microseconds that the
+ * integer ones save with rare interference (a burst every 25,000 spectra or so) against
+ * the plan, the extra launches and their partly filled waves, 25 to 40.  A million
+ * channel samples is 0.8 less (staged by words), a million DM terms 0.045 less from 32
+ * subbands on and 0.025 from 16 (fewer: the output bounds either); a replaced spectrum
+ * takes the items along whose windows reach it.  Measured, all items in FP32 and split:
+ * 30 k spectra of 256 channels to 40 DMs 80 and 100 us, 100 k of 1024 to 8 DMs 193 and
+ * 160, 300 k of 96 in 8 subbands to 500 277 and 301, 300 k of 1024 to 500 1521 and 950. */
+static bool dd_split_pays(const CsDedisp *D, const uint8_t *d_raw, long long nspec, long long nout)
+{
+    const bool words = ((dd_slab(D, false) * D->cps | D->nchan | (int)((uintptr_t)d_raw & 3)) & 3) == 0;
+    const double reach = std::min(1.0, (D->maxoff + D->halo + 256) / 25000.0);
+    const double sub = 1e-6 * nspec * D->nchan, dm = 1e-6 * nout * D->ndm * D->nsub;
+    const double ksub = !words ? -1.0 : D->halo > 512 ? 0.0 : 0.8;
+    const double kdm = (D->nsub >= 32 ? 0.045 : D->nsub >= 16 ? 0.025 : 0.0) * D->G / D->fG;
+    return sub * (ksub - reach) + dm * kdm * (1.0 - 0.5 * reach) >= 40.0;
+}
+
+/* The subband stage of one kind over the tiles up to sfill. */
+static cudaError_t dd_subbands(CsDedisp *D, dd::SubArgs sa, bool clip, long long sfill,
+                               cudaStream_t st)
+{
+    const int slab = dd_slab(D, clip);
     sa.slab = slab;
     sa.rowstride = sb_rowstride(D, slab);
     sa.table_off = sb_table_offset(D, slab);
@@ -1489,7 +1514,8 @@ static cudaError_t dd_enqueue(CsDedisp *D, const uint8_t *d_raw, long long nspec
     sa.L = D->L;
     sa.subf = D->d_subf;
     const bool ws = clip && D->fG > 0 && !getenv("CS_B200_DEDISP_ROUNDS");
-    const bool split = ws && D->gmax > 0 && D->d_clip != nullptr;
+    const bool split = ws && D->gmax > 0 && D->d_clip != nullptr &&
+                       dd_split_pays(D, d_raw, nspec, nout);
     cudaError_t e = cudaMemsetAsync(D->d_err, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     cudaEventRecord(D->ev0, st);
