@@ -725,7 +725,7 @@ struct GpuSession {
     f64k::Extra fx;
     f64k::Wide fw;
     int f64_wide;          /* search_f64_wide fits */
-    int f64_smem;
+    int f64_smem, f64_wide_smem;
     double *d_bcs, *d_scales;
     float4 *d_wt64;        /* search_f64_wide's weights */
     size_t c_wt64;
@@ -1543,7 +1543,7 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
             const int wide = f64k::wide_smem(w, x.ps_total);
             S->f64_wide = wide + (int)sizeof(CsHarm) * CS_MAX_NH <= S->max_smem &&
                           !getenv("CS_B200_GENERIC_KERNEL");
-            if (S->f64_wide) S->f64_smem = wide;
+            S->f64_wide_smem = wide;
         }
         CK(dev_reserve((void **)&S->d_bcs, &S->c_bcs, bcs.size() * sizeof(double)));
         CK(cudaMemcpyAsync(S->d_bcs, bcs.data(), bcs.size() * sizeof(double),
@@ -1557,7 +1557,6 @@ static int session_load(GpuSession *S, const FFTFile *ft, const SearchParams *p,
                 cudaSuccess) {
             (void)cudaGetLastError();
             S->f64_wide = 0;
-            S->f64_smem = f64k::smem_bytes(t.nh, x.ucols, x.prs, x.ps_total);
         }
         if (S->f64_wide && t.m == 16) {
             CK(cudaMemcpyAsync(S->d_wt64, t.Wt, (size_t)t.nrows * t.m * sizeof(float),
@@ -1838,6 +1837,16 @@ static wsk::Args ws_args(const GpuSession *S, const float2 *d_amps, double thres
     return w;
 }
 
+/* search_f64_wide, unless noise itself reaches the threshold (metrics are in sigmas:
+ * the best of a trial's some hundred windows is between 3 and 5) and the harmonics are
+ * few: its bound then decides nothing and its barriers are not hidden.  Kernels of
+ * 2^18 points, search_f64 and the wide one: nharms 7 at threshold 4 42 and 56 us, at 8 42
+ * and 24; nharms 16 at 4 136 and 140, at 8 136 and 62; nharms 24 at 4 269 and 224. */
+static bool f64_takes_wide(const GpuSession *S, double threshold)
+{
+    return S->f64_wide && (S->tab.nh > 16 || !(threshold < 6.0));
+}
+
 /* Enqueue the search of the spectrum at d_amps on S->st (no host sync). */
 static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double threshold,
                                   bool timed)
@@ -1866,10 +1875,11 @@ static cudaError_t enqueue_search(GpuSession *S, const float2 *d_amps, double th
         const int nsub = S->tab.ntiles * (CS_TILE_M / f64k::TT);
         const int grid = std::min(nsub, S->nsm);
         if (timed) cudaEventRecord(S->ev0, S->st);
-        if (S->f64_wide && S->tab.m == 16)
-            f64k::search_f64_wide<16><<<grid, f64k::WNT, S->f64_smem, S->st>>>(a64, x, S->fw);
-        else if (S->f64_wide)
-            f64k::search_f64_wide<0><<<grid, f64k::WNT, S->f64_smem, S->st>>>(a64, x, S->fw);
+        const bool wide = f64_takes_wide(S, threshold);
+        if (wide && S->tab.m == 16)
+            f64k::search_f64_wide<16><<<grid, f64k::WNT, S->f64_wide_smem, S->st>>>(a64, x, S->fw);
+        else if (wide)
+            f64k::search_f64_wide<0><<<grid, f64k::WNT, S->f64_wide_smem, S->st>>>(a64, x, S->fw);
         else if (S->tab.m == 16)
             f64k::search_f64<16><<<grid, f64k::NT, S->f64_smem, S->st>>>(a64, x);
         else
@@ -2125,7 +2135,7 @@ CS_EXPORT int cs_b200_session_info(const GpuSession *S, CsB200Info *info)
     info->nslot = S->tab.nslot;
     info->npad = S->tab.npad;
     info->kpad = S->tab.kpad;
-    info->smem_bytes = S->prec64 ? S->f64_smem : S->use_tma ? tma_smem(S->use_tma)
+    info->smem_bytes = S->prec64 ? (S->f64_wide ? S->f64_wide_smem : S->f64_smem) : S->use_tma ? tma_smem(S->use_tma)
                      : S->use_cols ? S->cols_smem
                      : S->use_ws ? ws_smem(S->use_ws) : smem_bytes(S->tab);
     info->grid = S->use_tma ? std::min(S->tx.nitems, S->nsm)

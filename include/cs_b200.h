@@ -39,8 +39,9 @@ int cs_b200_session_info(const GpuSession *s, CsB200Info *info);
 /* The kernel that a search of one finite spectrum by this session launches:
  * "search_cols", "search_ws" (a wave of tiles or less at few harmonics, or where
  * search_cols' geometry or memory does not fit),
- * "search_tma", "interp_tc + search_pre", "cs_search_kernel", "search_f64_wide" or
- * "search_f64" (a constant string). */
+ * "search_tma", "interp_tc + search_pre", "cs_search_kernel", "search_f64_wide" (at
+ * few harmonics and thresholds below 6 "search_f64") or "search_f64" (a constant
+ * string). */
 const char *cs_b200_session_kernel_name(const GpuSession *s);
 
 /* cs_gpu_session_create for sessions that are searched by cs_b200_multi_enqueue,

@@ -83,9 +83,10 @@ def _search(opts, N, amps, monkeypatch, generic, thresholds):
 def test_thresholds_below_single_metrics(gpu_ready, monkeypatch, nharms, fold, tone):
     N = 120000                                      # trials up to bin 960
     amps, rng = _noise(N, nharms)
+    amps *= 3                                       # metrics past 6: the wide kernel's
     tones = np.arange(301, 900, 31)                 # first harmonic on a tone, the others not
     for b in tones:
-        z = tone * np.exp(6.28j * rng.random())
+        z = 3 * tone * np.exp(6.28j * rng.random())
         amps[2 * b:2 * b + 2] = z.real, z.imag
     opts = Options(nharms=nharms, blocksize=1000, precision=1)
     every = _search(opts, N, amps, monkeypatch, True, [-1e30])[0]
@@ -96,8 +97,8 @@ def test_thresholds_below_single_metrics(gpu_ready, monkeypatch, nharms, fold, t
     for a in range(0, sel.size - 64, 64):
         if near[a:a + 64].all():
             tops.append(sel["metric"][a:a + 64].max())
-    tops = np.sort(tops)[:60]                       # the tone cancelled in the fold
-    thr = np.sort(tops[tops > 0]) * (1 - 1e-6)
+    tops = np.sort(tops)                            # the least: the tone cancelled in the fold
+    thr = tops[tops > 6.1][:60] * (1 - 1e-6)
     assert thr.size >= 12
     new = _search(opts, N, amps, monkeypatch, False, thr)
     old = _search(opts, N, amps, monkeypatch, True, thr)
@@ -133,3 +134,26 @@ def test_values_fp32_sums_do_not_hold(gpu_ready, monkeypatch, value):
         np.testing.assert_array_equal(a["nharm"], b["nharm"])
         top = b["metric"].max() if b.size else 0.0
         np.testing.assert_allclose(a["metric"], b["metric"], rtol=1e-9, atol=1e-9 * top)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("threshold", [4.0, 8.0])
+def test_few_harmonics_are_not_slower_than_search_f64(gpu_ready, monkeypatch, threshold):
+    """Where noise reaches the threshold the bound is of no use."""
+    N = 1 << 18
+    amps, _ = _noise(N, 1)
+    opts = Options(nharms=7, precision=1, threshold=threshold)
+    took = []
+    for generic in (True, False):
+        if generic:
+            monkeypatch.setenv("CS_B200_GENERIC_KERNEL", "1")
+        ses = Session(N, 64e-6, opts)
+        monkeypatch.delenv("CS_B200_GENERIC_KERNEL", raising=False)
+        ses.run_raw(amps)
+        ms = []
+        for _ in range(15):
+            ses.enqueue(None)
+            ms.append(ses.collect()[1])
+        ses.close()
+        took.append(float(np.median(ms)))
+    assert took[1] < 1.15 * took[0]
