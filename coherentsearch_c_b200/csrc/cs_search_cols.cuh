@@ -25,7 +25,7 @@
  * every other one 1.5 %: the host runs the kernel for any geometry instead.)
  *
  * Measured: 8.05 M trials at nharms 60 4.68 -> 2.31 ms, 1.0 M 0.70 -> 0.336, 3.0 M
- * at 32 0.474 -> 0.331, 1.1 M at 16 0.219 -> 0.152.  No unit is full (issue slots
+ * at 32 0.474 -> 0.331, 1.1 M at 16 0.219 -> 0.142.  No unit is full (issue slots
  * 63 % busy, 70 % on the fullest scheduler; shared-memory path 47 %, FP32 44 %): at
  * nharms 60 a third of an interpolation warp's time goes into waits for boxes, 60
  * small ones a tile (8 rows of some 200 bytes, 175 cycles each as it runs; 8

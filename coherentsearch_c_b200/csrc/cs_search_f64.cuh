@@ -240,9 +240,11 @@ search_f64(const SearchArgs args, const Extra ex)
  *            maximum, which does not depend on the split.
  * The additions of a chain, the differences and the final expression are
  * search_f64's; only the DFT's summation is grouped by the matrix instruction
- * (1e-16 of a profile bin).  Bound by the DFT and the latency of the two serial
- * stages.  N = 2^19, nharms 60: 0.86 ms against 3.30.  It needs room for X beside the
- * prefix sums; geometries that only fit without it take search_f64. */
+ * (1e-16 of a profile bin).  Bound by the latency of the serial stages and the
+ * barriers between them: some 16 k cycles a sub-tile, 3.7 k of them the DFT's
+ * arithmetic.  N = 2^19, nharms 60: 0.86 ms against 3.30.  It needs room for X beside the
+ * prefix sums; geometries that only fit without it take search_f64, as do few
+ * harmonics at low thresholds. */
 constexpr int WNT = 512, NW = WNT / 32;
 constexpr int XS = TT + 4;          /* X row stride (doubles): fragment rows hit all banks */
 
