@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(256) pad_amax_kernel(const float2 *__restrict_
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < namps; i += gridDim.x * blockDim.x) {
         const float2 a = amps[i];
         pad[FRONT + i] = a;
-        const float v = fmaxf(fabsf(a.x), fabsf(a.y));
-        if (!(v <= 3.0e38f)) bad = 1;       /* NaN or Inf */
-        mx = fmaxf(mx, v);
+        mx = fmaxf(mx, fmaxf(fabsf(a.x), fabsf(a.y)));
+        /* NaN or Inf, each by itself: a maximum hides a NaN */
+        if (!(fabsf(a.x) <= 3.0e38f) || !(fabsf(a.y) <= 3.0e38f)) bad = 1;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

@@ -42,3 +42,24 @@ def test_same_bits_as_search_ws(gpu_ready, monkeypatch, nharms, hidr, value):
     for new, old in zip(*out):
         for f in ("r", "metric", "nharm"):
             np.testing.assert_array_equal(new[f], old[f])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("at", [0, 1, 199, 30006])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_one_component_alone(gpu_ready, monkeypatch, at, value):
+    """Beside a finite other component, which a maximum of the two would show."""
+    N = 65536
+    rng = np.random.default_rng(at)
+    amps = (rng.standard_normal(2 * (N // 2)) * np.sqrt(0.5)).astype(np.float32)
+    amps[at] = value
+    out = []
+    for ws in (False, True):
+        if ws:
+            monkeypatch.setenv("CS_B200_WS_KERNEL", "1")
+        ses = Session(N, 64e-6, Options(threshold=3.0))
+        out.append(np.sort(ses.run_raw(amps), order=["r", "nharm"]))
+        ses.close()
+    assert out[1].size > 100
+    for f in ("r", "metric", "nharm"):
+        np.testing.assert_array_equal(out[0][f], out[1][f])
