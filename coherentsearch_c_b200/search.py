@@ -156,7 +156,7 @@ class Session:
             C.byref(self.ft), C.byref(self.params), C.byref(self.plans), self._cs, self.total,
             self.opts.blocksize, self.nchunks, self.r_lo, self.lodr, device)
         if not self.sess:
-            raise RuntimeError("session_create failed (see stderr)")
+            raise RuntimeError("cs_gpu_session_create failed (see stderr)")
 
     def info(self) -> nt.CsB200Info:
         inf = nt.CsB200Info()
