@@ -1129,6 +1129,18 @@ static int sb_smem(const CsDedisp *D, int slab, bool clip = false)
     return sb_flag_offset(D, slab) + (clip ? dd::SB_TT + D->halo : 0);
 }
 
+/* Raise a kernel's dynamic shared memory to what the device allows beside its static
+ * one.  The limit is the kernel's, not a plan's: set to one plan's need it would refuse
+ * the launches of an earlier plan that needs more. */
+static cudaError_t dd_smem_cap(const void *fn, int max_optin)
+{
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                max_optin - (int)fa.sharedSizeBytes);
+}
+
 CS_EXPORT CsDedisp *cs_dedisp_create(int nchan, int nsub, int ndm, const int *idispdt,
                                      const int *offsets, int spectra_per_subint,
                                      int blocks_per_read, long long max_spectra, int device)
@@ -1342,8 +1354,7 @@ CS_EXPORT CsDedisp *cs_dedisp_create(int nchan, int nsub, int ndm, const int *id
         DDCK(cudaMalloc((void **)&D->d_fgbytes, sizeof(int) * fgbytes.size()));
         DDCK(cudaMemcpy(D->d_fgbytes, fgbytes.data(), sizeof(int) * fgbytes.size(),
                         cudaMemcpyHostToDevice));
-        DDCK(cudaFuncSetAttribute(dd::dd_dms_f32_ws, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  4 * D->fnstage * D->fstage_words));
+        DDCK(dd_smem_cap((const void *)dd::dd_dms_f32_ws, max_optin));
     }
     DDCK(cudaMalloc((void **)&D->d_err, sizeof(int)));
     DDCK(cudaMemset(D->d_err, 0, sizeof(int)));
@@ -1377,8 +1388,7 @@ CS_EXPORT CsDedisp *cs_dedisp_create(int nchan, int nsub, int ndm, const int *id
     DDCK(cudaEventCreate(&D->ev1));
     DDCK(cudaEventCreate(&D->ev2));
     if (G > 0)
-        DDCK(cudaFuncSetAttribute(dd::dd_dms_u16, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  4 * D->nstage * D->stage_words));
+        DDCK(dd_smem_cap((const void *)dd::dd_dms_u16, max_optin));
     DDCK(cudaFuncSetAttribute(dd::dd_subband_u8, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               max_optin));
     DDCK(cudaFuncSetAttribute(dd::dd_subband_u8_256<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
