@@ -918,9 +918,10 @@ __global__ void __launch_bounds__(FD_THREADS, 1) dd_dms_f32_ws(const FdArgs a)
 /* Which items of a clipped run need FP32                            */
 /* ---------------------------------------------------------------- */
 /* A sum without a replaced spectrum in it is a sum of integers below 2^24: the
- * FP32 result in any order, and what the integer stages give.  So a clipped run
- * takes the FP32 stages only for the DM items whose windows reach a flagged
- * spectrum, and the integer stages for the rest.  Interference is rare: 12
+ * FP32 result in any order, and what the integer stages give.  So a clipped run that
+ * is large enough (dd_split_pays) takes the FP32 stages only for the DM items whose
+ * windows reach a flagged spectrum, and the integer stages for the rest.  Interference
+ * is rare: 12
  * bursts in 300 k spectra leave 8 % of the items, and the two stages took 1165 +
  * 383 us in FP32 where they take 612 + 121 us and 90 + 104 us now.  When every spectrum is flagged the
  * integer stages have no items. */

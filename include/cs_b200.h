@@ -139,7 +139,9 @@ int cs_b200_session_collapse_wait(GpuSession *s, CandidateList *out, float *kern
  * overlap another's kernel, and a slot's device buffers are reused across
  * lengths.  A slot takes a request only while the device memory that all
  * slots hold stays within `mem_budget` bytes (0: no limit); idle slots give
- * their buffers back when another slot needs the room. */
+ * their buffers back when another slot needs the room.  What only makes a search
+ * faster (a second copy of the spectrum and tables) is held where the budget leaves
+ * room for it. */
 typedef struct CsBatch CsBatch;
 
 CsBatch *cs_gpu_batch_create(int device, int nslots, size_t mem_budget);
